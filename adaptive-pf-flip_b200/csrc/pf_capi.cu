@@ -1,5 +1,6 @@
 // pf_capi.cu -- the extern "C" entry points of libpfgpu (include/pfgpu.h):
 // context set-up, particle exchange, grid access and the solver-step calls.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -60,7 +61,7 @@ void free_all(pf_ctx* c) {
   for (int* p : c->scan_levels) F(p);
   F(c->d_scalar);
   F(c->x); F(c->r); F(c->p); F(c->Ap); F(c->diag); F(c->cx); F(c->cy); F(c->cz); F(c->kind); F(c->z_plain);
-  F(c->partials); F(c->ctl); F(c->ctl_outer); F(c->nbr_plain);
+  F(c->partials); F(c->ctl); F(c->ctl_outer); F(c->nbr_plain); F(c->ps_entries);
   F(c->xf); F(c->rf); F(c->pf32); F(c->Apf); F(c->diagf); F(c->cxf); F(c->cyf); F(c->czf); F(c->pbf); F(c->cbf);
   F(c->b64);
   F(c->d_clamp); F(c->d_flags); F(c->cell_flags); F(c->esc_buf); F(c->mk_first); F(c->rc_buf);
@@ -93,6 +94,7 @@ int create_impl(pf_ctx* ctx, const pf_grid_desc* d) {
   if (prop.major < 10) return set_error(ctx, PF_ERR_NO_DEVICE, "libpfgpu needs an sm_100 device");
   ctx->device = d->device;
   ctx->num_sms = prop.multiProcessorCount;
+  ctx->smem_optin = prop.sharedMemPerBlockOptin;
   PF_CUDA_TRY(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   PF_CUDA_TRY(cudaEventCreate(&ctx->ev0));
   PF_CUDA_TRY(cudaEventCreate(&ctx->ev1));
@@ -202,6 +204,17 @@ int create_impl(pf_ctx* ctx, const pf_grid_desc* d) {
   // per-CTA partials: up to kRedSlots doubles per reduction CTA
   PF_CUDA_TRY(cudaMalloc(&ctx->partials, (size_t)kMaxRedBlocks * kRedSlots * sizeof(double)));
   PF_CUDA_TRY(cudaMalloc(&ctx->nbr_plain, (cells / PF_TV + 1) * 6 * sizeof(int)));
+  {
+    // one block: the persistent solvers' entries, their arrival counter (a line
+    // of its own), and the faces of every slot of a system whose vectors stay
+    // on chip: six of 64 values, two sets
+    const size_t nf = 2 * (size_t)std::min(nt, (size_t)kMaxRedBlocks) * 6 * 64;
+    const size_t n = kPsEntries + 8 + nf;
+    PF_CUDA_TRY(cudaMalloc(&ctx->ps_entries, n * sizeof(PsPair)));
+    PF_CUDA_TRY(cudaMemset(ctx->ps_entries, 0, n * sizeof(PsPair)));
+    ctx->ps_counter = (unsigned long long*)(ctx->ps_entries + kPsEntries);
+    ctx->ps_faces = ctx->ps_entries + kPsEntries + 8;
+  }
   PF_CUDA_TRY(cudaMalloc(&ctx->ctl, sizeof(SolveCtl)));
   PF_CUDA_TRY(cudaMemset(ctx->ctl, 0, sizeof(SolveCtl)));
   PF_CUDA_TRY(cudaMallocHost(&ctx->h_ctl, sizeof(SolveCtl)));

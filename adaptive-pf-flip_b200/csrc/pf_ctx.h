@@ -90,6 +90,13 @@ struct pf_ctx {
   double *x = nullptr, *r = nullptr, *p = nullptr, *Ap = nullptr;
   double *diag = nullptr, *cx = nullptr, *cy = nullptr, *cz = nullptr;
   double* partials = nullptr;  // [kMaxRedBlocks * 4]
+  // persistent solvers (pf_persist.cuh): published entries and arrival counter,
+  // the tile faces they hand over (two sets), and the last tag used
+  pf::PsPair* ps_entries = nullptr;
+  unsigned long long* ps_counter = nullptr;
+  pf::PsPair* ps_faces = nullptr;
+  unsigned long long ps_tag = 0;
+  size_t smem_optin = 0;       // shared memory a CTA of this device may use
   int* nbr_plain = nullptr;    // [cells_cap / 512 * 6] neighbour slots of each pooled tile (PLAIN PCG)
   double* z_plain = nullptr;   // [cells_cap] PLAIN PCG's z (r / diag), from its update to its direction pass
   uint8_t* kind = nullptr;     // per cell: 0 not an unknown, 1 fluid, 2 pinned
@@ -222,7 +229,10 @@ int ensure_back_set(pf_ctx* ctx);
 // 11 along the normal axis and 10 along each transverse axis (float2 each).
 constexpr int kSplatStageTile = 3 * 11 * 10 * 10;
 
-constexpr int kMaxRedBlocks = 1184;  // 8 CTAs per SM on 148 SMs
+constexpr int kPsGrid = 148;         // CTAs of a persistent solver (one per SM)
+// entries of the persistent solvers (pf_persist.cuh): two reductions' sums and
+// one's maxima, each in two sets
+constexpr size_t kPsEntries = 4 * (size_t)kMaxRedBlocks + 2 * kPsGrid;
 constexpr int kRedSlots = 4;         // partial values one reduction CTA may write
 
 // pf_timing.cu

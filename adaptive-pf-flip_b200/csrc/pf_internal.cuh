@@ -134,6 +134,14 @@ struct SolveCtl {
   double flex[2];          // flexible PCG: r.D^-1 r and r.z_prev of the current residual
 };
 
+constexpr int kMaxRedBlocks = 1184;  // 8 CTAs per SM on 148 SMs
+
+// A value published with the tag of its reduction (pf_persist.cuh).
+struct alignas(16) PsPair {
+  double value;
+  unsigned long long tag;
+};
+
 // Programmatic dependent launch.  A kernel started by launch_pdl may begin
 // while its predecessor on the stream is still running: it calls pdl_wait()
 // before it touches memory the predecessor writes (the wait returns once the

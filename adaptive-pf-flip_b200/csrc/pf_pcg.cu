@@ -1,8 +1,11 @@
 // pf_pcg.cu -- pressure solvers over the pool-layout 7-point system.
 //
 // PLAIN: FP64 Jacobi-PCG with the reference's recurrences and stopping rule
-//   (src/driver/sparse_ops3d_tp.cpp:315-364); three kernels per iteration:
-//   SpMV + p.Ap, x/r update + r.z + max|r|, direction update.
+//   (src/driver/sparse_ops3d_tp.cpp:315-364).  Systems of up to about 7200 tiles
+//   run in a persistent kernel (pf_persist.cu); larger ones, and the
+//   allocation-free projection, take three kernels per iteration: SpMV + p.Ap,
+//   x/r update + r.z + max|r|, direction update.  There the 139 bytes a cell and
+//   iteration bound the time (0.51 ms at 256^3, 0.70 of the copy bandwidth).
 // MIXED: FP64 outer iterative refinement r = b - A x with the exact FP64
 //   operator, inner Jacobi-PCG with FP32 vectors and FP32 (or BF16) scaled
 //   face coefficients, FP64 inner products and norms.  The BF16 operator keeps
@@ -355,7 +358,10 @@ int pcg_plain(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, PcgVec<dou
   vec.z = ctx->z_plain;
   if (nslots > 0)
     (++ctx->launches), k_plain_nbr<<<nblocks((size_t)6 * nslots, 256), 256, 0, ctx->stream>>>(G, nslots, ctx->nbr_plain);
-  while (!c.done && launched < cfg->max_iter) {
+  bool ran = false;
+  rc = plain_persist(ctx, nslots, kind, ctx->nbr_plain, vec, scale, cfg->max_iter, &c, &ran);
+  if (rc) return rc;
+  while (!ran && !c.done && launched < cfg->max_iter) {
     const int nb = std::min(batch, cfg->max_iter - launched);
     for (int q = 0; q < nb; ++q) {
       (++ctx->launches), k_spmv_plain_tab<<<nred, PF_TV, 0, ctx->stream>>>(nslots, ctx->ctl, kind, ctx->nbr_plain, vec,

@@ -17,7 +17,8 @@
 // reproducible run to run).  Each reduction finishes in the last CTA of the
 // producing kernel, which also advances the scalar recurrences (alpha, beta,
 // convergence) in device memory; the host only polls a done flag every few
-// iterations.
+// iterations.  Systems that fit a persistent grid run all of that in one launch
+// with the same sums (pf_persist.cu).
 #include <cmath>
 
 #include "pf_ctx.h"
@@ -150,8 +151,10 @@ __global__ void __launch_bounds__(PF_TV) k_assemble(DevGrid G, int nslots, Solve
       rz = __dadd_rn(rz, __dmul_rn(rr, z));
       rmax = fmax(rmax, fabs(rr));
       vec.store_p(o, z);
+      if (vec.z) vec.z[o] = (V)z;
     } else {
       vec.store_p(o, 0.0);
+      if (vec.z) vec.z[o] = (V)0.0;
     }
     vec.diag[o] = (V)dg;
     vec.cx[o] = (V)clx;
@@ -262,7 +265,9 @@ int project(pf_ctx* ctx, const pf_phase* ph, double dt, const pf_solve_cfg* cfg,
   const double scale = dt / (ctx->g.dx * ctx->g.dx);
   PF_CUDA_TRY(cudaEventRecord(ctx->ev0, ctx->stream));
   SolveResult res{};
-  PcgVec<double> vec{ctx->x, ctx->r, ctx->p, ctx->Ap, ctx->diag, ctx->cx, ctx->cy, ctx->cz};
+  // PLAIN starts from z = r / diag as well as from the first direction
+  PcgVec<double> vec{ctx->x, ctx->r, ctx->p, ctx->Ap, ctx->diag, ctx->cx, ctx->cy, ctx->cz,
+                     cfg->mode == PF_SOLVER_PLAIN ? ctx->z_plain : nullptr};
   (++ctx->launches), k_assemble<double><<<nred, PF_TV, 0, ctx->stream>>>(G, nslots, ctx->ctl, kind, vec, scale, cfg->c_div, phk,
                                                       ctx->partials);
   PF_CUDA_TRY(cudaGetLastError());

@@ -13,7 +13,7 @@ namespace pf {
 template <typename V>
 struct PcgVec {
   V *x, *r, *p, *Ap, *diag, *cx, *cy, *cz;
-  V* z;  // PLAIN: z = r / diag from the update to the direction pass (null: formed in both)
+  V* z;  // PLAIN: z = r / diag from the assembly and the update to the direction pass (null: formed in both)
   __device__ __forceinline__ void store_p(size_t o, double v) const { p[o] = (V)v; }
 };
 
@@ -288,6 +288,10 @@ int solve_inner_outer(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, co
 // solver drivers (pf_pcg.cu)
 int pcg_plain(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, PcgVec<double> vec, double scale,
               const pf_solve_cfg* cfg, SolveResult* res);
+// PLAIN as a persistent kernel (pf_persist.cu); *ran is false when the system
+// has too many slots for it, and nothing was done
+int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, PcgVec<double> v, double scale,
+                  int max_iter, SolveCtl* out, bool* ran);
 int solve_mixed(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, double scale, const pf_solve_cfg* cfg,
                 const void* phase_consts, SolveResult* res);
 int ensure_solver_buffers(pf_ctx* ctx, int mode);

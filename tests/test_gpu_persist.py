@@ -1,0 +1,92 @@
+"""The PLAIN solve at every way its work is split over the GPU.
+
+A system's tiles go to 148 CTAs: one to eight tiles each live on chip (a kernel
+per count, 5 and 7 running in the next larger one's), more are streamed with as
+many of r and x on chip as fit, and beyond about 7200 tiles three kernels run
+per iteration.  The grids below take one of each, ragged ones among them, with
+solid, empty and fluid cells mixed.
+
+A few iterations are compared with the oracle's: both round every vector update
+alike in FP64 and differ in the order of the inner products only, which moves
+the iterate by some 1e-15 per iteration; the pressure is stored in FP32, so it
+may differ by one unit in its last place (2^-23 of the value), and where a value
+cancels by 1e-12 of the field's scale.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+from gpu_helpers import to_oracle_phase
+
+pytestmark = pytest.mark.gpu
+
+GRIDS = [(5, 6, 4), (39, 30, 22), (46, 47, 40), (54, 55, 62), (63, 62, 56), (64, 64, 64), (70, 71, 72), (78, 79, 72),
+         (80, 79, 77), (88, 86, 81), (104, 97, 90), (127, 118, 100)]
+
+
+def _system(shape, seed):
+    nx, ny, nz = shape
+    rng = np.random.default_rng(seed)
+    mk = np.full((nz, ny, nx), 2, np.float32)
+    inner = rng.choice(np.array([0, 1, 1, 1, 1, 1, 1, 2], np.float32), (nz - 2, ny - 2, nx - 2))
+    mk[1:-1, 1:-1, 1:-1] = inner
+    f = {7: mk}
+    for a, s in enumerate(((nz, ny, nx + 1), (nz, ny + 1, nx), (nz + 1, ny, nx))):
+        f[a] = rng.normal(0, 1, s).astype(np.float32)
+        f[3 + a] = (rng.uniform(0, 1.2, s) * (rng.random(s) > 0.2)).astype(np.float32)
+    return f
+
+
+@pytest.mark.parametrize("shape", GRIDS, ids=str)
+def test_iterates_match_the_oracle(pf, shape):
+    its, dt, c_div = 9, 1.0 / 60, 0.01
+    fields = _system(shape, sum(shape))
+    pp = pf.PhaseParams(1.0, 0.01)
+    g = pf.SparseMacGrid3D(*shape, 1.0 / max(shape), max_particles=int(np.prod(shape)) // 4 + 64)
+    og = O.OracleGrid(*shape, 1.0 / max(shape))
+    for f, v in fields.items():
+        act = np.ones(g.bdims(f)[::-1], np.uint8)
+        g.set_field(f, v, act)
+        og.set_field(f, v, act)
+    st = pf.spProjectStepVC3D(g, pp, dt, its, 0.0, c_div)
+    so = O.Oracle().project(og, to_oracle_phase(pp), dt, its, 0.0, c_div)
+    assert st.iterations == so.iterations == its and not st.converged
+    assert st.n_cells == so.n_cells and st.pin_cell == so.pin_cell
+    assert abs(st.res_final - so.res_final) <= 1e-11 * so.res_final
+    p, q = g.get_field(pf.PF_P)[0].astype(np.float64), og.get_field(pf.PF_P)[0].astype(np.float64)
+    scale = np.abs(q).max()
+    assert scale > 0
+    assert np.all(np.abs(p - q) <= 2.0 ** -23 * np.abs(q) + 1e-12 * scale)
+    g.close()
+
+
+def test_launches_chain_bit_for_bit(pf):
+    """A solve of more iterations than one launch runs (2048), against the
+    allocation-free entry point, whose three kernels per iteration form the
+    same sums in the same order: the same iterations and the same bits."""
+    import ctypes as C
+
+    import torch
+    n = 30  # 64 tiles, all pooled by both entry points
+    fields = _system((n, n, n), 5)
+    fields[7][1:-1, 1:-1, 1:-1] = 1  # every interior cell fluid, one pinned
+    for a in range(3):  # a thousandfold contrast in two halves
+        m = fields[3 + a]
+        m[:] = np.where(np.arange(m.shape[1])[None, :, None] < n // 2, 2.0, 0.0)
+    pp, dt, its = pf.PhaseParams(1.0, 0.0001), 1.0 / 60, 2500
+    g = pf.SparseMacGrid3D(n, n, n, 1.0 / n, max_particles=4096)
+    for f, v in fields.items():
+        g.set_field(f, v, np.ones(g.bdims(f)[::-1], np.uint8))
+    st = pf.spProjectStepVC3D(g, pp, dt, its, 0.0)
+    dev = {k: torch.from_numpy(fields[f]).cuda() for k, f in
+           (("mk", 7), ("mu", 3), ("mv", 4), ("mw", 5), ("u", 0), ("v", 1), ("w", 2))}
+    p = torch.zeros((n, n, n), device="cuda")
+    s2 = pf._lib.SolveStats()
+    torch.cuda.synchronize()
+    rc = pf.load().pf_project_noalloc(n, n, n, 1.0 / n, *[dev[k].data_ptr() for k in ("mk", "mu", "mv", "mw", "u", "v", "w")],
+                                      p.data_ptr(), C.byref(pp._c()), dt, its, 0.0, 0.0, 0.0, C.byref(s2), None)
+    assert rc == 0
+    assert st.iterations == s2.iterations and st.breakdown == s2.breakdown
+    assert st.res_final == s2.res_final
+    assert np.array_equal(g.get_field(pf.PF_P)[0], p.cpu().numpy())
+    g.close()
