@@ -16,9 +16,6 @@
 namespace pf {
 namespace {
 
-constexpr int kPsFace = 6 * 64;  // face values of a slot
-constexpr int kPsChunk = 2048;   // iterations per launch
-
 struct PsPlain {
   int nslots, nred;
   SolveCtl* ctl;
@@ -30,54 +27,6 @@ struct PsPlain {
   PsBar bar;
   PsPair* faces;  // [2][nslots][6][64]
   unsigned long long tag;
-};
-
-// index of the cell that face value q (0..63) of face d touches: the
-// neighbour's boundary cell
-__device__ __forceinline__ int halo_cell(int d, int q) {
-  const int a = q & 7, b = q >> 3;
-  switch (d) {
-    case 0: return (a << 3) | (b << 6);          // +x neighbour, its x = 0
-    case 1: return 7 | (a << 3) | (b << 6);
-    case 2: return a | (b << 6);                 // +y neighbour, its y = 0
-    case 3: return a | 56 | (b << 6);
-    case 4: return a | (b << 3);
-    default: return a | (b << 3) | 448;
-  }
-}
-
-// The scalars of a solve, advanced alike by every thread of the grid (the
-// rules of finalize_stage, kStagePAp and kStageUpdate).
-struct PsScalars {
-  double alpha, beta, rz, res, tol;
-  int it, max_iter, done;
-  __device__ __forceinline__ explicit PsScalars(const SolveCtl* c)
-      : alpha(0.0), beta(c->beta), rz(c->rz), res(c->res), tol(c->tol), it(c->it), max_iter(c->max_iter),
-        done(c->done) {}
-  __device__ __forceinline__ void after_pap(double S) {
-    if (!isfinite(S)) done = 4;
-    else if (fabs(S) < 1e-30 || !isfinite(rz / S)) done = 2;
-    else alpha = rz / S;
-  }
-  __device__ __forceinline__ void after_update(double S, double M) {
-    it += 1;
-    res = M;
-    if (!isfinite(M) || !isfinite(S)) done = 4;
-    else if (M < tol) done = 1;
-    else if (it >= max_iter) done = 3;
-    else {
-      beta = S / rz;
-      rz = S;
-    }
-  }
-  __device__ __forceinline__ void store(SolveCtl* c) const {
-    c->alpha = alpha;
-    c->beta = beta;
-    c->rz = rz;
-    c->res = res;
-    c->it = it;
-    c->done = done;
-  }
 };
 
 // r / d, correctly rounded, from inv = RN(1 / d) formed once per solve: the
@@ -524,7 +473,7 @@ int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
   if (!resident && k * ps_slot_bytes() > room) return PF_OK;
   PsPlain a{nslots, std::min(nslots, kMaxRedBlocks), ctx->ctl, kind, nbr, v.x, v.r, v.p, v.z, v.diag, v.cx, v.cy,
             v.cz, scale, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0};
-  *ran = true;
+  *ran = max_iter > 0;
   for (int launched = 0; !out->done && launched < max_iter; launched += kPsChunk) {
     a.tag = ctx->ps_tag + 1;
     ctx->ps_tag += kPsChunk;

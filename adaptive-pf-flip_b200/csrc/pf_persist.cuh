@@ -43,6 +43,8 @@ namespace pf {
 constexpr int kPsVirt = kMaxRedBlocks / kPsGrid;    // virtual CTAs of one CTA, at most
 constexpr unsigned kPsPolls = 1u << 22;
 constexpr int kPsWarps = PF_TV / 32;                // warps of a virtual CTA
+constexpr int kPsFace = 6 * 64;                     // face values of a slot
+constexpr int kPsChunk = 2048;                      // iterations per launch
 
 static_assert(kMaxRedBlocks % kPsGrid == 0, "a CTA must own whole virtual CTAs");
 static_assert(kPsWarps == 16, "half a warp folds one virtual CTA");
@@ -242,5 +244,53 @@ __device__ __forceinline__ bool ps_wait(PsShared& sh, const PsBar& bar, int whic
   if (kMax) M = warp_max_nonneg(sh.gmax[lane & 7]);
   return !dead;
 }
+
+// index of the cell that face value q (0..63) of face d touches: the
+// neighbour's boundary cell
+__device__ __forceinline__ int halo_cell(int d, int q) {
+  const int a = q & 7, b = q >> 3;
+  switch (d) {
+    case 0: return (a << 3) | (b << 6);          // +x neighbour, its x = 0
+    case 1: return 7 | (a << 3) | (b << 6);
+    case 2: return a | (b << 6);                 // +y neighbour, its y = 0
+    case 3: return a | 56 | (b << 6);
+    case 4: return a | (b << 3);
+    default: return a | (b << 3) | 448;
+  }
+}
+
+// The scalars of a solve, advanced alike by every thread of the grid (the
+// rules of finalize_stage, kStagePAp and kStageUpdate).
+struct PsScalars {
+  double alpha, beta, rz, res, tol;
+  int it, max_iter, done;
+  __device__ __forceinline__ explicit PsScalars(const SolveCtl* c)
+      : alpha(0.0), beta(c->beta), rz(c->rz), res(c->res), tol(c->tol), it(c->it), max_iter(c->max_iter),
+        done(c->done) {}
+  __device__ __forceinline__ void after_pap(double S) {
+    if (!isfinite(S)) done = 4;
+    else if (fabs(S) < 1e-30 || !isfinite(rz / S)) done = 2;
+    else alpha = rz / S;
+  }
+  __device__ __forceinline__ void after_update(double S, double M) {
+    it += 1;
+    res = M;
+    if (!isfinite(M) || !isfinite(S)) done = 4;
+    else if (M < tol) done = 1;
+    else if (it >= max_iter) done = 3;
+    else {
+      beta = S / rz;
+      rz = S;
+    }
+  }
+  __device__ __forceinline__ void store(SolveCtl* c) const {
+    c->alpha = alpha;
+    c->beta = beta;
+    c->rz = rz;
+    c->res = res;
+    c->it = it;
+    c->done = done;
+  }
+};
 
 }  // namespace pf

@@ -292,6 +292,10 @@ int pcg_plain(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, PcgVec<dou
 // has too many slots for it, and nothing was done
 int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, PcgVec<double> v, double scale,
                   int max_iter, SolveCtl* out, bool* ran);
+// MIXED's inner solve (started by k_mixed_start) as a persistent kernel
+// (pf_persist_mixed.cu); *ran as above
+int mixed_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, float* e, float* r, const float* d,
+                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, SolveCtl* out, bool* ran);
 int solve_mixed(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, double scale, const pf_solve_cfg* cfg,
                 const void* phase_consts, SolveResult* res);
 int ensure_solver_buffers(pf_ctx* ctx, int mode);
