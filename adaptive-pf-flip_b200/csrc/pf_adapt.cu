@@ -603,15 +603,26 @@ __global__ void __launch_bounds__(kNT) k_particle_reduce(PSet P, int n, double V
   }
 }
 
-// the partials in a fixed order (one thread: kRedBlocks values)
-__global__ void k_particle_reduce_total(const double* part, int nb, double* out) {
-  double vmax = 0.0, vol = 0.0;
-  for (int b = 0; b < nb; ++b) {
+// the partials in a fixed order.  The volumes are added one after the other, as
+// a chain of kRedBlocks additions; every load is done before it starts (one
+// thread that loads as it adds waits for memory at each step: 93 us against 8).
+__global__ void __launch_bounds__(kNT) k_particle_reduce_total(const double* part, double* out) {
+  __shared__ double vol[kRedBlocks], wmax[kNT / 32];
+  double vmax = 0.0;
+  for (int b = threadIdx.x; b < kRedBlocks; b += kNT) {
     vmax = fmax(vmax, part[2 * b]);
-    vol = __dadd_rn(vol, part[2 * b + 1]);
+    vol[b] = part[2 * b + 1];
   }
+  for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = vmax;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double v = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < kRedBlocks; ++b) v = __dadd_rn(v, vol[b]);
+  for (int w = 0; w < kNT / 32; ++w) vmax = fmax(vmax, wmax[w]);
   out[0] = vmax;
-  out[1] = vol;
+  out[1] = v;
 }
 
 // SparseSim3DTP::applyParticleAdaptivity (src/driver/sparse_sim3d_tp.cpp:843-848)
@@ -647,7 +658,7 @@ int step_controls(pf_ctx* ctx, double dt, double Vp, const pf_step_controls& c, 
   double* out = reinterpret_cast<double*>(s->d_stats + 8);  // two doubles in the 16-int statistics buffer
   const int nb = kRedBlocks;
   (++ctx->launches), k_particle_reduce<<<nb, kNT, 0, ctx->stream>>>(particles_of(ctx), n, Vp, part);
-  (++ctx->launches), k_particle_reduce_total<<<1, 1, 0, ctx->stream>>>(part, nb, out);
+  (++ctx->launches), k_particle_reduce_total<<<1, kNT, 0, ctx->stream>>>(part, out);
   PF_CUDA_TRY(cudaGetLastError());
   PF_CUDA_TRY(cudaMemcpyAsync(s->h_ctl, out, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   PF_CUDA_TRY(cudaEventRecord(s->ctl_ev, ctx->stream));

@@ -190,16 +190,68 @@ __global__ void k_assign_slots(uint8_t* need, const int* flags, const int* rank,
 
 __global__ void k_bump_nslots(int* d_nslots, const int* added) { *d_nslots += *added; }
 
+// The four steps above (flags, scan, slots, new size) in one CTA for tile
+// lattices of up to kCommitTiles tiles (152^3 cells): thread t takes tiles
+// kCommitPer t ..., so the scan keeps ascending tile order.  A commit is a chain
+// of six to eight launches of about 2.4 us otherwise, four times a step.
+constexpr int kCommitNT = 1024, kCommitPer = 8, kCommitTiles = kCommitNT * kCommitPer;
+__global__ void __launch_bounds__(kCommitNT) k_commit_small(uint8_t* need, int* tile_slot, int* slot_tile,
+                                                            int* d_nslots, int n) {
+  __shared__ int warp_tot[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, t0 = threadIdx.x * kCommitPer;
+  unsigned fresh = 0;
+#pragma unroll
+  for (int q = 0; q < kCommitPer; ++q)
+    if (t0 + q < n && need[t0 + q]) {
+      if (tile_slot[t0 + q] < 0) fresh |= 1u << q;
+      need[t0 + q] = 0;
+    }
+  const int mine = __popc(fresh);
+  int x = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_tot[wid] = x;
+  const int base = *d_nslots;
+  __syncthreads();
+  if (wid == 0) {
+    int w = warp_tot[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    warp_tot[lane] = w;
+  }
+  __syncthreads();
+  int s = base + (wid > 0 ? warp_tot[wid - 1] : 0) + x - mine;
+#pragma unroll
+  for (int q = 0; q < kCommitPer; ++q)
+    if ((fresh >> q) & 1u) {
+      tile_slot[t0 + q] = s;
+      slot_tile[s] = t0 + q;
+      ++s;
+    }
+  if (threadIdx.x == 0) *d_nslots = base + warp_tot[31];
+}
+
 int pool_commit(pf_ctx* ctx) {
   const int n = ctx->g.ntiles;
   int* flags = ctx->tile_new;
   int* rank = ctx->tile_rank;
-  (++ctx->launches), k_need_flags<<<nblocks(n, 256), 256, 0, ctx->stream>>>(ctx->tile_need, ctx->tile_slot, flags, n);
-  int rc = scan_exclusive(ctx, flags, rank, n, ctx->d_scalar);
-  if (rc) return rc;
-  (++ctx->launches), k_assign_slots<<<nblocks(n, 256), 256, 0, ctx->stream>>>(ctx->tile_need, flags, rank, ctx->tile_slot,
-                                                          ctx->slot_tile, ctx->d_nslots, n);
-  (++ctx->launches), k_bump_nslots<<<1, 1, 0, ctx->stream>>>(ctx->d_nslots, ctx->d_scalar);
+  if (n <= kCommitTiles) {
+    (++ctx->launches), k_commit_small<<<1, kCommitNT, 0, ctx->stream>>>(ctx->tile_need, ctx->tile_slot, ctx->slot_tile,
+                                                                        ctx->d_nslots, n);
+  } else {
+    (++ctx->launches), k_need_flags<<<nblocks(n, 256), 256, 0, ctx->stream>>>(ctx->tile_need, ctx->tile_slot, flags, n);
+    int rc = scan_exclusive(ctx, flags, rank, n, ctx->d_scalar);
+    if (rc) return rc;
+    (++ctx->launches), k_assign_slots<<<nblocks(n, 256), 256, 0, ctx->stream>>>(
+        ctx->tile_need, flags, rank, ctx->tile_slot, ctx->slot_tile, ctx->d_nslots, n);
+    (++ctx->launches), k_bump_nslots<<<1, 1, 0, ctx->stream>>>(ctx->d_nslots, ctx->d_scalar);
+  }
   PF_CUDA_TRY(cudaGetLastError());
   PF_CUDA_TRY(cudaMemcpyAsync(ctx->h_nslots, ctx->d_nslots, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   PF_CUDA_TRY(cudaEventRecord(ctx->pool_ev, ctx->stream));

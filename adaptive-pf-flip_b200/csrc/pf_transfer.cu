@@ -11,7 +11,7 @@
 //
 // P2G design (replaces the reference's 8 colour threads that each rescan every
 // particle): particles are binned by cell (tile-major) with warp-aggregated
-// atomics; one CTA per tile splats its particles, one thread per cell holding
+// atomics; one CTA per tile (or per tile and face field) splats its particles, one thread per cell holding
 // a register window per face field, into warp-private shared boxes, combines
 // them into a staging box per tile, and the normalisation pass sums the
 // staging boxes that reach each node.  Every sum runs in a fixed order, so
@@ -247,8 +247,8 @@ __global__ void k_mark_particles(DevGrid G, const float* __restrict__ px, const 
 //
 // Determinism.  Every node's sum is formed in one fixed order, so two runs on
 // the same particles give bit-identical fields:
-//   * a cell's particles are taken in ascending index (sorted at the start of
-//     the kernel; binning ranks particles in arrival order);
+//   * a cell's particles are taken in ascending index (sorted by
+//     k_cell_sort; binning ranks particles in arrival order);
 //   * each warp adds its 32 cells' windows into a shared box of its own, one
 //     window offset at a time (the lanes address distinct nodes);
 //   * the 16 warp boxes of the tile are combined node by node in warp order
@@ -714,32 +714,14 @@ __device__ __forceinline__ unsigned long long splat_field(const DevGrid& G, floa
   return box;
 }
 
-// The tile's 4x4x4 block box: node-block (o >> 2) relative to the tile's first
-// 4^3 block minus one, i.e. box index 0 is the block below the tile.
-__global__ void __launch_bounds__(kSplatThreads, 3) k_splat(DevGrid G, const int* __restrict__ cell_start,
-                                                           int* __restrict__ perm, int* __restrict__ sort_tmp,
-                                                           float2* __restrict__ stage,
-                                                           const float* __restrict__ px,
-                                                           const float* __restrict__ py,
-                                                           const float* __restrict__ pz,
-                                                           const float* __restrict__ vx,
-                                                           const float* __restrict__ vy,
-                                                           const float* __restrict__ vz,
-                                                           const uint8_t* __restrict__ type,
-                                                           const float* __restrict__ vol, float m_l, float m_g) {
-  extern __shared__ float2 wbox[];  // [kSplatGroups][kWarpBox]
-  __shared__ unsigned sblk[6];      // [3 axes][64 reached blocks of the box]
+// A tile's particles in ascending index per cell, by the whole CTA: small cells
+// in registers, larger ones by counted ranks.  sv: kBigSortStage ints.
+__device__ __forceinline__ void sort_cells(const int* __restrict__ cs, int* perm, int* sort_tmp, int* sv) {
   __shared__ int nbig;
   __shared__ int big[PF_TV];
-  const int t = blockIdx.x;
-  const int* cs = cell_start + (size_t)t * PF_TV;
-  if (cs[0] >= cs[PF_TV]) return;
   const int tid = threadIdx.x;
-  if (tid < 6) sblk[tid] = 0u;
   if (tid == 0) nbig = 0;
   __syncthreads();
-  // cells in ascending particle index: small cells in registers, larger ones
-  // by ranks counted by the whole CTA
   for (int pass = 0; pass < kSplatPasses; ++pass) {
     const int cl = splat_cell_of(tid, pass);
     const int beg = cs[cl], n = cs[cl + 1] - beg;
@@ -752,7 +734,6 @@ __global__ void __launch_bounds__(kSplatThreads, 3) k_splat(DevGrid G, const int
   for (int b = 0; b < nbig; ++b) {
     const int cl = big[b];
     const int beg = cs[cl], n = cs[cl + 1] - beg;
-    int* sv = reinterpret_cast<int*>(wbox);
     const bool staged = n <= kBigSortStage;
     if (staged)
       for (int i = tid; i < n; i += kSplatThreads) sv[i] = perm[beg + i];
@@ -770,6 +751,37 @@ __global__ void __launch_bounds__(kSplatThreads, 3) k_splat(DevGrid G, const int
     for (int i = tid; i < n; i += kSplatThreads) perm[beg + i] = sort_tmp[beg + i];
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(kSplatThreads) k_cell_sort(const int* __restrict__ cell_start, int* perm,
+                                                             int* sort_tmp) {
+  extern __shared__ int sort_stage[];
+  const int* cs = cell_start + (size_t)blockIdx.x * PF_TV;
+  if (cs[0] < cs[PF_TV]) sort_cells(cs, perm, sort_tmp, sort_stage);
+}
+
+// kPerField: one CTA per tile and face field, the particles sorted before
+// (k_cell_sort); else one CTA per tile sorts them and takes the fields in turn.
+template <bool kPerField>
+__global__ void __launch_bounds__(kSplatThreads, 3) k_splat(DevGrid G, const int* __restrict__ cell_start,
+                                                           int* __restrict__ perm, int* __restrict__ sort_tmp,
+                                                           float2* __restrict__ stage,
+                                                           const float* __restrict__ px,
+                                                           const float* __restrict__ py,
+                                                           const float* __restrict__ pz,
+                                                           const float* __restrict__ vx,
+                                                           const float* __restrict__ vy,
+                                                           const float* __restrict__ vz,
+                                                           const uint8_t* __restrict__ type,
+                                                           const float* __restrict__ vol, float m_l, float m_g) {
+  extern __shared__ float2 wbox[];  // [kSplatGroups][kWarpBox]
+  __shared__ unsigned sblk[6];      // [3 axes][64 reached blocks of the box]
+  const int t = kPerField ? blockIdx.x / 3 : blockIdx.x, field = kPerField ? blockIdx.x - 3 * t : -1;
+  const int* cs = cell_start + (size_t)t * PF_TV;
+  if (cs[0] >= cs[PF_TV]) return;
+  const int tid = threadIdx.x;
+  if (tid < 6) sblk[tid] = 0u;
+  if (!kPerField) sort_cells(cs, perm, sort_tmp, reinterpret_cast<int*>(wbox));
   const int tx = t % G.g.TX, tq = t / G.g.TX, ty = tq % G.g.TY, tz = tq / G.g.TY;
   const int t0[3] = {tx * 8, ty * 8, tz * 8};
   const double inv_dx = G.g.inv_dx;
@@ -779,16 +791,20 @@ __global__ void __launch_bounds__(kSplatThreads, 3) k_splat(DevGrid G, const int
   const bool edge = tx == 0 || ty == 0 || tz == 0 || tx * 8 + 10 > G.g.nx || ty * 8 + 10 > G.g.ny ||
                     tz * 8 + 10 > G.g.nz;
   float2* st = stage + (size_t)t * kStageTile;
-  unsigned long long box[3];
-  box[0] = splat_field<0>(G, wbox, st, cs, perm, px, py, pz, vx, type, vol, m_l, m_g, t0, inv_dx, inv_dx_f, fast,
-                          edge);
-  box[1] = splat_field<1>(G, wbox, st, cs, perm, px, py, pz, vy, type, vol, m_l, m_g, t0, inv_dx, inv_dx_f, fast,
-                          edge);
-  box[2] = splat_field<2>(G, wbox, st, cs, perm, px, py, pz, vz, type, vol, m_l, m_g, t0, inv_dx, inv_dx_f, fast,
-                          edge);
+  unsigned long long box[3] = {0ull, 0ull, 0ull};
+  if (!kPerField || field == 0)
+    box[0] = splat_field<0>(G, wbox, st, cs, perm, px, py, pz, vx, type, vol, m_l, m_g, t0, inv_dx, inv_dx_f, fast,
+                            edge);
+  if (!kPerField || field == 1)
+    box[1] = splat_field<1>(G, wbox, st, cs, perm, px, py, pz, vy, type, vol, m_l, m_g, t0, inv_dx, inv_dx_f, fast,
+                            edge);
+  if (!kPerField || field == 2)
+    box[2] = splat_field<2>(G, wbox, st, cs, perm, px, py, pz, vz, type, vol, m_l, m_g, t0, inv_dx, inv_dx_f, fast,
+                            edge);
   // one shared OR per warp and word
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
+    if (kPerField && a != field) continue;
     const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)box[a]);
     const unsigned hi = __reduce_or_sync(0xffffffffu, (unsigned)(box[a] >> 32));
     if ((tid & 31) == 0) {
@@ -797,7 +813,9 @@ __global__ void __launch_bounds__(kSplatThreads, 3) k_splat(DevGrid G, const int
     }
   }
   __syncthreads();
-  // activity bytes of the reached blocks (a byte is stored only when it reads 0)
+  // activity bytes of the reached blocks (a byte is stored only when it reads
+  // 0).  The tile's 4x4x4 block box: node-block (o >> 2) relative to the tile's
+  // first 4^3 block minus one, i.e. box index 0 is the block below the tile.
   for (int e = tid; e < 3 * 64; e += kSplatThreads) {
     const int a = e >> 6, idx = e & 63;
     if ((sblk[2 * a + (idx >> 5)] >> (idx & 31)) & 1u) {
@@ -1078,11 +1096,11 @@ constexpr int kG2PBox3 = kG2PBox * kG2PBox * kG2PBox;
 
 __global__ void __launch_bounds__(256) k_g2p_tiles(DevGrid G, const int* __restrict__ cell_start,
                                                    const int* __restrict__ perm, ParticlePtrs P, double aL,
-                                                   double aG) {
+                                                   double aG, int split) {
   __shared__ float2 box[3][kG2PBox3];  // (current, saved)
-  const int t = blockIdx.x;
+  const int t = blockIdx.x / split, part = blockIdx.x - t * split;
   const int beg = cell_start[(size_t)t * PF_TV], end = cell_start[(size_t)(t + 1) * PF_TV];
-  if (beg >= end) return;
+  if (beg + part * (int)blockDim.x >= end) return;
   const int tx = t % G.g.TX, tq = t / G.g.TX, ty = tq % G.g.TY, tz = tq / G.g.TY;
   const int b0 = tx * 8 - 1, b1 = ty * 8 - 1, b2 = tz * 8 - 1;
   // the pool slots of the 27 tiles around this one: the box's nodes (clamped
@@ -1114,7 +1132,8 @@ __global__ void __launch_bounds__(256) k_g2p_tiles(DevGrid G, const int* __restr
   const bool fast = G.g.dx_pow2 && G.g.ox == 0.0 && G.g.oy == 0.0 && G.g.oz == 0.0;
   const float inv_dx_f = (float)G.g.inv_dx;
   // the next particle's attributes are loaded while this one is sampled
-  int q = beg + threadIdx.x;
+  const int step = split * blockDim.x;
+  int q = beg + part * blockDim.x + threadIdx.x;
   int pn = 0;
   float xn = 0.0f, yn = 0.0f, zn = 0.0f, vn[3] = {0.0f, 0.0f, 0.0f};
   uint8_t tn = 0;
@@ -1123,12 +1142,12 @@ __global__ void __launch_bounds__(256) k_g2p_tiles(DevGrid G, const int* __restr
     xn = P.px[pn]; yn = P.py[pn]; zn = P.pz[pn]; tn = P.type[pn];
     vn[0] = P.vx[pn]; vn[1] = P.vy[pn]; vn[2] = P.vz[pn];
   }
-  for (; q < end; q += blockDim.x) {
+  for (; q < end; q += step) {
     const int p = pn;
     const float X = xn, Y = yn, Z = zn, v0[3] = {vn[0], vn[1], vn[2]};
     const uint8_t ty = tn;
-    if (q + (int)blockDim.x < end) {
-      pn = perm[q + blockDim.x];
+    if (q + step < end) {
+      pn = perm[q + step];
       xn = P.px[pn]; yn = P.py[pn]; zn = P.pz[pn]; tn = P.type[pn];
       vn[0] = P.vx[pn]; vn[1] = P.vy[pn]; vn[2] = P.vz[pn];
     }
@@ -1339,13 +1358,14 @@ __device__ __forceinline__ void box_velocity(const DevGrid& G, const float2 (*bo
 
 __global__ void __launch_bounds__(256, 3) k_g2p_advect_tiles(DevGrid G, const int* __restrict__ cell_start,
                                                           const int* __restrict__ perm, ParticlePtrs P, double dt,
-                                                          int order, double aL, double aG, int* counters) {
+                                                          int order, double aL, double aG, int* counters,
+                                                          int split) {
   __shared__ float2 box[3][kAdvBox3];  // (current, saved)
   __shared__ int nslot[27];
   __shared__ int tally[8];
-  const int t = blockIdx.x;
+  const int t = blockIdx.x / split, part = blockIdx.x - t * split;
   const int beg = cell_start[(size_t)t * PF_TV], end = cell_start[(size_t)(t + 1) * PF_TV];
-  if (beg >= end) return;
+  if (beg + part * (int)blockDim.x >= end) return;
   const int tx = t % G.g.TX, tq = t / G.g.TX, ty = tq % G.g.TY, tz = tq / G.g.TY;
   const int b0 = tx * 8 - 2, b1 = ty * 8 - 2, b2 = tz * 8 - 2;
   if (threadIdx.x < 27) {
@@ -1381,7 +1401,8 @@ __global__ void __launch_bounds__(256, 3) k_g2p_advect_tiles(DevGrid G, const in
   const double hi[3] = {G.g.ox + (G.g.nx - 0.5) * G.g.dx, G.g.oy + (G.g.ny - 0.5) * G.g.dx,
                         G.g.oz + (G.g.nz - 0.5) * G.g.dx};
   unsigned cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int q = beg + threadIdx.x;
+  const int step = split * blockDim.x;
+  int q = beg + part * blockDim.x + threadIdx.x;
   int pn = 0;
   float xn = 0.0f, yn = 0.0f, zn = 0.0f, vn[3] = {0.0f, 0.0f, 0.0f};
   uint8_t tn = 0;
@@ -1390,12 +1411,12 @@ __global__ void __launch_bounds__(256, 3) k_g2p_advect_tiles(DevGrid G, const in
     xn = P.px[pn]; yn = P.py[pn]; zn = P.pz[pn]; tn = P.type[pn];
     vn[0] = P.vx[pn]; vn[1] = P.vy[pn]; vn[2] = P.vz[pn];
   }
-  for (; q < end; q += blockDim.x) {
+  for (; q < end; q += step) {
     const int p = pn;
     const float X = xn, Y = yn, Z = zn, v0[3] = {vn[0], vn[1], vn[2]};
     const uint8_t ptype = tn;
-    if (q + (int)blockDim.x < end) {
-      pn = perm[q + blockDim.x];
+    if (q + step < end) {
+      pn = perm[q + step];
       xn = P.px[pn]; yn = P.py[pn]; zn = P.pz[pn]; tn = P.type[pn];
       vn[0] = P.vx[pn]; vn[1] = P.vy[pn]; vn[2] = P.vz[pn];
     }
@@ -1537,15 +1558,34 @@ __global__ void k_calib_contrib(double mp, double* contrib) {
   contrib[q] = v;
 }
 
-__global__ void k_calib_sum(const double* contrib, double rho_l, double* out) {
+__global__ void __launch_bounds__(512) k_calib_sum(const double* contrib, double rho_l, double* out) {
+  __shared__ double v[4096];
+  for (int q = threadIdx.x; q < 4096; q += blockDim.x) v[q] = contrib[q];
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   double s = 0.0;
-  for (int q = 0; q < 4096; ++q) s = __dadd_rn(s, contrib[q]);
+#pragma unroll 16
+  for (int q = 0; q < 4096; ++q) s = __dadd_rn(s, v[q]);
   *out = s > 0.0 ? __ddiv_rn(s, rho_l) : 1.0;
 }
 
 ParticlePtrs particle_ptrs(pf_ctx* ctx) {
   return ParticlePtrs{ctx->px, ctx->py, ctx->pz, ctx->vx, ctx->vy, ctx->vz, ctx->vol, ctx->type};
 }
+
+// Grids of few tiles give a tile more than one CTA.  A CTA of the splat or of
+// the tile-staged G2P fills a third of an SM, so up to about 3 x 148 tiles the
+// GPU is one short wave; past that the work repeated per CTA costs more than the
+// fuller SMs give.  Measured on filled / 0.7-filled boxes, ms before and after:
+//   P2G, one CTA per tile and face field: 20^3 (27 tiles) 0.074 -> 0.036, 40^3
+//     (216) 0.096 / 0.091 -> 0.063 / 0.056, 48^3 (343) 0.115 / 0.110 -> 0.090 /
+//     0.083, 56^3 (512) 0.120 / 0.119 -> 0.119 / 0.095, 72^3 (1000) 0.208 -> 0.220,
+//     128^3 (4913) 1.079 -> 1.134;
+//   G2P + advection, two CTAs per tile: 20^3 0.063 -> 0.044, 48^3 0.080 / 0.070
+//     -> 0.061 / 0.056, 56^3 0.085 -> 0.092, 128^3 0.576 -> 0.662 (three CTAs are
+//     slower than two from 48^3 on).
+bool splat_per_field(const pf_ctx* ctx) { return ctx->g.ntiles <= 4 * ctx->num_sms; }
+int tile_split(const pf_ctx* ctx) { return ctx->g.ntiles <= 3 * ctx->num_sms ? 2 : 1; }
 
 int slot_grid(const pf_ctx* ctx) { return slot_blocks(ctx, 16 * ctx->num_sms); }
 
@@ -1626,9 +1666,18 @@ static int p2g_core(pf_ctx* ctx, const pf_phase* ph, double Vp) {
   {
     StageScope sc(ctx, PF_STAGE_SPLAT);
     const size_t smem = (size_t)kSplatGroups * kWarpBox * sizeof(float2);
-    (++ctx->launches), k_splat<<<nt, kSplatThreads, smem, ctx->stream>>>(
-        dev_grid(ctx), ctx->tile_start, ctx->perm, ctx->prank, ctx->splat_stage, ctx->px, ctx->py, ctx->pz, ctx->vx,
-        ctx->vy, ctx->vz, ctx->type, ctx->vol, (float)(ph->rho_l * Vp), (float)(ph->rho_g * Vp));
+    const float ml = (float)(ph->rho_l * Vp), mg = (float)(ph->rho_g * Vp);
+    if (splat_per_field(ctx)) {
+      (++ctx->launches), k_cell_sort<<<nt, kSplatThreads, kBigSortStage * sizeof(int), ctx->stream>>>(
+          ctx->tile_start, ctx->perm, ctx->prank);
+      (++ctx->launches), k_splat<true><<<3 * nt, kSplatThreads, smem, ctx->stream>>>(
+          dev_grid(ctx), ctx->tile_start, ctx->perm, ctx->prank, ctx->splat_stage, ctx->px, ctx->py, ctx->pz, ctx->vx,
+          ctx->vy, ctx->vz, ctx->type, ctx->vol, ml, mg);
+    } else {
+      (++ctx->launches), k_splat<false><<<nt, kSplatThreads, smem, ctx->stream>>>(
+          dev_grid(ctx), ctx->tile_start, ctx->perm, ctx->prank, ctx->splat_stage, ctx->px, ctx->py, ctx->pz, ctx->vx,
+          ctx->vy, ctx->vz, ctx->type, ctx->vol, ml, mg);
+    }
     ctx->splat_fresh = true;
     PF_CUDA_TRY(cudaGetLastError());
   }
@@ -1693,8 +1742,8 @@ int g2p(pf_ctx* ctx, const pf_ctx* saved, double aL, double aG) {
   } else {
     if (!ctx->saved_valid) return set_error(ctx, PF_ERR_INVALID, "g2p: no saved velocity (call pf_save_velocity)");
     if (ctx->bins_valid)
-      (++ctx->launches), k_g2p_tiles<<<ctx->g.ntiles, 256, 0, ctx->stream>>>(G, ctx->tile_start, ctx->perm,
-                                                                               particle_ptrs(ctx), aL, aG);
+      (++ctx->launches), k_g2p_tiles<<<ctx->g.ntiles * tile_split(ctx), 256, 0, ctx->stream>>>(
+          G, ctx->tile_start, ctx->perm, particle_ptrs(ctx), aL, aG, tile_split(ctx));
     else
       (++ctx->launches), k_g2p<false><<<nblocks(n, 256), 256, 0, ctx->stream>>>(G, G, particle_ptrs(ctx), n, aL, aG);
   }
@@ -1760,8 +1809,9 @@ int g2p_advect(pf_ctx* ctx, double aL, double aG, double dt, int order, pf_clamp
   PF_CUDA_TRY(cudaMemsetAsync(ctx->d_clamp, 0, 8 * sizeof(int), ctx->stream));
   if (n > 0) {
     if (ctx->bins_valid && !esc_flags)
-      (++ctx->launches), k_g2p_advect_tiles<<<ctx->g.ntiles, 256, 0, ctx->stream>>>(
-          dev_grid(ctx), ctx->tile_start, ctx->perm, particle_ptrs(ctx), dt, order, aL, aG, ctx->d_clamp);
+      (++ctx->launches), k_g2p_advect_tiles<<<ctx->g.ntiles * tile_split(ctx), 256, 0, ctx->stream>>>(
+          dev_grid(ctx), ctx->tile_start, ctx->perm, particle_ptrs(ctx), dt, order, aL, aG, ctx->d_clamp,
+          tile_split(ctx));
     else
       (++ctx->launches), k_advect<<<nblocks(n, 256), 256, 0, ctx->stream>>>(dev_grid(ctx), particle_ptrs(ctx), n, dt,
                                                                              order, ctx->d_clamp, esc_flags, 1, aL, aG);
@@ -1776,7 +1826,7 @@ int calibrate(pf_ctx* ctx, const pf_phase* ph, double Vp, double* out) {
   double* contrib = (double*)ctx->staging;  // 4096 doubles + 1
   const double mp = ph->rho_l * Vp;
   (++ctx->launches), k_calib_contrib<<<16, 256, 0, ctx->stream>>>(mp, contrib);
-  (++ctx->launches), k_calib_sum<<<1, 1, 0, ctx->stream>>>(contrib, ph->rho_l, contrib + 4096);
+  (++ctx->launches), k_calib_sum<<<1, 512, 0, ctx->stream>>>(contrib, ph->rho_l, contrib + 4096);
   PF_CUDA_TRY(cudaGetLastError());
   PF_CUDA_TRY(cudaMemcpyAsync(out, contrib + 4096, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
