@@ -32,8 +32,10 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
+#include "pf_persist.cuh"
 #include "pf_solver.cuh"
 
 namespace pf {
@@ -830,6 +832,177 @@ __global__ void __launch_bounds__(kMrNT) k_mr_update(int N, MrVecs V, MrCtl* ctl
   mr_reduce(rz, num, bad, rmax, partials, ctl, kMrUpdate);
 }
 
+// The whole PCG as one persistent kernel (pf_persist.cuh) for systems of up to
+// kMrResRows rows per thread of 148 CTAs: a thread keeps its rows' x, r, z, p,
+// diagonal and slice position in registers, and only p goes through memory, for
+// the neighbours' gathers:
+//   direction  p = z + beta p               barrier that hands over p
+//   SpMV       Ap, p.Ap                     reduction A
+//   update     x, r, z, r.z, max|r|         reduction B (and one for r.(z - z_prev)
+//                                           with the flexible beta)
+// The columns and coefficients are kept in shared memory, whole slices as far as
+// they fit, so a row waits for one round of gathers instead of two.  As two
+// launches per iteration with last-CTA reductions, an iteration of the 128^3 dam
+// break (142k rows) took 19 us; here 9.1, two thirds of it the three barriers.
+// The scalar rules are mr_finalize's, applied by every thread to its own copy;
+// the inner products add up in another fixed order.
+constexpr int kMrResNT = 1024, kMrResRows = 3;
+
+template <int R>
+__global__ void __launch_bounds__(kMrResNT, 1) k_mr_pcg(int N, const int* __restrict__ slice_ptr,
+                                                      const int* __restrict__ col, const double* __restrict__ coef,
+                                                      MrVecs V, MrCtl* ctl_g, const int* air, int first, PsBar bar,
+                                                      unsigned long long tag0, int* dead, int cap) {
+  extern __shared__ double s_coef[];  // [cap], then the columns [cap]
+  __shared__ PsShared sh;
+  __shared__ int s_at[R * (kMrResNT / 32)];  // each slice's length, then its place (-1: not kept)
+  int* s_col = reinterpret_cast<int*>(s_coef + cap);
+  const int pin = mr_pin(air, N);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  MrCtl ctl = *ctl_g;
+  if (first) ctl.beta = 0.0;
+  // slices go to the CTAs in turn: the wide rows (coarse cells beside fine ones,
+  // up to 24 terms) are neighbours in the numbering, and one CTA's share of a
+  // contiguous split kept the others waiting (10.5 us an iteration)
+  const int r0 = (wid * kPsGrid + (int)blockIdx.x) * 32 + lane, stride = kPsGrid * kMrResNT;
+  double x[R], rr[R], z[R], p[R], dg[R], ap[R];
+  int base[R], width[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const int r = r0 + j * stride;
+    x[j] = rr[j] = z[j] = p[j] = dg[j] = ap[j] = 0.0;
+    base[j] = width[j] = 0;
+    if (r < N) {
+      x[j] = V.x[r];
+      rr[j] = V.r[r];
+      z[j] = V.z[r];
+      p[j] = V.p[r];
+      dg[j] = V.diag[r];
+      const int a = slice_ptr[r >> 5];
+      base[j] = a + (r & 31);
+      width[j] = r == pin ? 0 : (slice_ptr[(r >> 5) + 1] - a) >> 5;
+    }
+  }
+  // a warp's 32 rows are one slice per j
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const int w = (int)__reduce_max_sync(0xffffffffu, (unsigned)width[j]);
+    if (lane == 0) s_at[j * (kMrResNT / 32) + wid] = 32 * w;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int used = 0;
+    for (int q = 0; q < R * (kMrResNT / 32); ++q) {
+      const int len = s_at[q];
+      s_at[q] = used + len <= cap ? used : -1;
+      if (used + len <= cap) used += len;
+    }
+  }
+  __syncthreads();
+  int at[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    at[j] = s_at[j * (kMrResNT / 32) + wid];
+    if (at[j] >= 0)
+      for (int t = 0; t < width[j]; ++t) {
+        s_coef[at[j] + 32 * t + lane] = coef[base[j] + 32 * t];
+        s_col[at[j] + 32 * t + lane] = col[base[j] + 32 * t];
+      }
+    at[j] += at[j] >= 0 ? lane : 0;
+  }
+  bool alive = true;
+  unsigned long long arrivals = 0;
+  auto reduce = [&](auto with_max, double v, double m, int which, int parity, unsigned long long tag, double& S,
+                    double& M) {
+    constexpr bool kMax = decltype(with_max)::value;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (kMax) m = warp_max_nonneg(m);
+    if (lane == 0) {
+      sh.loc[wid >> 4][wid & 15] = v;
+      if (kMax) sh.wmax[wid] = m;
+    }
+    ps_publish<kMax>(sh, bar, which, parity, tag, kMrResNT / PF_TV);
+    arrivals += gridDim.x;
+    return ps_wait<kMax>(sh, bar, which, parity, tag, kPsGrid * (kMrResNT / PF_TV), arrivals, S, M,
+                         [] { return true; });
+  };
+  for (int turn = 0; turn < kPsChunk && !ctl.done; ++turn) {
+    const int par = turn & 1;
+    const unsigned long long tag = tag0 + 2 * turn;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int r = r0 + j * stride;
+      p[j] = z[j] + ctl.beta * p[j];
+      if (r < N) V.p[r] = p[j];
+    }
+    arrivals += gridDim.x;
+    alive = ps_barrier(bar, arrivals);
+    if (!alive) break;
+    double pap = 0.0, S = 0.0, M = 0.0;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      double off = 0.0;
+      const bool kept = at[j] >= 0;
+      const double* cf = kept ? s_coef + at[j] : coef + base[j];
+      const int* cl = kept ? s_col + at[j] : col + base[j];
+      constexpr int kG = 8;  // gathers in flight
+      for (int t = 0; t < width[j]; t += kG) {
+        double pv[kG];
+#pragma unroll
+        for (int u = 0; u < kG; ++u) pv[u] = t + u < width[j] ? __ldcg(V.p + cl[32 * (t + u)]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kG; ++u)
+          if (t + u < width[j]) off += cf[32 * (t + u)] * pv[u];
+      }
+      const int r = r0 + j * stride;
+      ap[j] = r == pin ? p[j] : dg[j] * p[j] - off;
+      if (r < N) pap += p[j] * ap[j];
+    }
+    alive = reduce(std::false_type{}, pap, 0.0, 0, par, tag, S, M);
+    if (!alive) break;
+    mr_finalize(&ctl, kMrPAp, S, 0.0, 0.0, 0.0);
+    if (ctl.done) break;
+    double rz = 0.0, num = 0.0, rmax = 0.0;
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      if (r0 + j * stride >= N) continue;
+      x[j] += ctl.alpha * p[j];
+      rr[j] -= ctl.alpha * ap[j];
+      bad = bad || !isfinite(x[j]) || !isfinite(rr[j]);
+      if (isfinite(rr[j])) rmax = fmax(rmax, fabs(rr[j]));
+      const double zn = (ctl.jacobi && dg[j] > 0.0) ? rr[j] / dg[j] : rr[j];
+      rz += rr[j] * zn;
+      if (ctl.flexible) num += rr[j] * (zn - z[j]);
+      z[j] = zn;
+    }
+    // a value that is not finite ends the solve: it travels as a NaN maximum
+    // (the largest bit pattern), and the finite maximum follows
+    const double finite_max = rmax;
+    if (bad) rmax = __longlong_as_double(0x7ff8000000000000ll);
+    alive = reduce(std::true_type{}, rz, rmax, 1, par, tag, S, M);
+    if (!alive) break;
+    const double s0 = S, nonfinite = isnan(M) ? 1.0 : 0.0;
+    double s1 = 0.0, dummy = 0.0;
+    if (nonfinite != 0.0) alive = reduce(std::true_type{}, 0.0, finite_max, 1, par ^ 1, tag + 1, dummy, M);
+    else if (ctl.flexible) alive = reduce(std::false_type{}, num, 0.0, 0, par ^ 1, tag + 1, s1, dummy);
+    if (!alive) break;
+    mr_finalize(&ctl, kMrUpdate, s0, s1, nonfinite, M);
+  }
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const int r = r0 + j * stride;
+    if (r >= N) continue;
+    V.x[r] = x[j];
+    if (ctl.done) continue;  // else the next launch goes on from here
+    V.r[r] = rr[j];
+    V.z[r] = z[j];
+  }
+  if (r0 == 0 && alive) *ctl_g = ctl;
+  if (!alive && threadIdx.x == 0) *dead = 1;
+}
+
 __global__ void k_mr_ctl_init(MrCtl* ctl, int max_iter, double abs_tol, double rel_tol, int jacobi, int flexible,
                               int adaptive, double growth) {
   *ctl = MrCtl{};
@@ -1352,7 +1525,38 @@ int project_mr(pf_ctx* ctx, MrState* s, const pf_mr_step_cfg* cfg, pf_mr_step_st
   MrCtl c{};
   int launched = 0;
   stage_begin(ctx, PF_STAGE_PCG);
-  while (true) {
+  const int rows = (N + kPsGrid * kMrResNT - 1) / (kPsGrid * kMrResNT);
+  const bool resident = rows <= kMrResRows && ctx->num_sms >= kPsGrid && cfg->cg_iters > 0;
+  if (resident) {
+    int* dead = s->counters + 8;
+    // room for the slices: what the device gives a CTA less the static arrays
+    const size_t smem = (ctx->smem_optin - sizeof(PsShared) - kMrResRows * (kMrResNT / 32) * sizeof(int) - 256) & ~(size_t)63;
+    int cap = (int)(smem / (sizeof(double) + sizeof(int)));
+    cap &= ~31;
+    PF_CUDA_TRY(cudaMemsetAsync(dead, 0, sizeof(int), ctx->stream));
+    PsBar bar{ctx->ps_entries, ctx->ps_counter};
+    for (int first = 1; !c.done && launched < cfg->cg_iters; first = 0) {
+      unsigned long long tag = ctx->ps_tag + 1;
+      ctx->ps_tag += 2 * kPsChunk;
+      PF_CUDA_TRY(cudaMemsetAsync(ctx->ps_counter, 0, sizeof(unsigned long long), ctx->stream));
+      int n = N, f = first;
+      const int *sp = s->slice_ptr, *cl = s->col, *ar = tot + 3;
+      const double* cf = s->coef;
+      void* args[] = {&n, &sp, &cl, &cf, &V, &s->ctl, &ar, &f, &bar, &tag, &dead, &cap};
+      const void* kernel = rows == 1 ? (const void*)k_mr_pcg<1> : rows == 2 ? (const void*)k_mr_pcg<2>
+                                                                            : (const void*)k_mr_pcg<3>;
+      PF_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      ++ctx->launches;
+      PF_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(kPsGrid), dim3(kMrResNT), args, smem, ctx->stream));
+      PF_CUDA_TRY(cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(MrCtl), cudaMemcpyDeviceToHost, ctx->stream));
+      PF_CUDA_TRY(cudaMemcpyAsync(s->h_ints + 4, dead, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+      if (s->h_ints[4]) return set_error(ctx, PF_ERR_CUDA, "multires pressure solve: a grid-wide wait ran out");
+      c = *s->h_ctl;
+      launched += kPsChunk;
+    }
+  }
+  while (!resident) {
     PF_CUDA_TRY(cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(MrCtl), cudaMemcpyDeviceToHost, ctx->stream));
     PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     c = *s->h_ctl;

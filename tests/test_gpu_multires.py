@@ -167,5 +167,33 @@ def test_mr_dynamic_refinement_matches_oracle(pf):
     sim.close()
 
 
+@pytest.mark.parametrize("n,flexible", [((60, 60, 57), False), ((76, 72, 73), True)])
+def test_mr_large_system_iterates_match_oracle(pf, n, flexible):
+    """Systems of more rows than 148 CTAs have threads (two and three rows a
+    thread), a few PCG iterations.  P2G's velocities agree within about 1e-6 of
+    the field's scale, and a CG iterate of a handful of iterations passes the
+    right-hand side's error on with a small factor: 1e-4 bounds it."""
+    dx = 1.0 / 64
+    s = MRSettings(dt=1 / 60, phase=_phase(), dynamic_refinement=False, cg_flexible_beta=flexible, cg_iters=6,
+                   cg_rel_tol=0.0, cg_tol=0.0)
+    rng = np.random.default_rng(n[0])
+    k, j, i = np.meshgrid(np.arange(1, n[2] - 1), np.arange(1, n[1] - 6), np.arange(1, n[0] - 1), indexing="ij")
+    cells = np.stack([i.ravel(), j.ravel(), k.ravel()], 1)
+    pos = ((cells + rng.uniform(0.1, 0.9, cells.shape)) * dx).astype(np.float32)
+    vel = rng.normal(0, 0.3, pos.shape).astype(np.float32)
+    typ = np.zeros(len(pos), np.uint8)
+    # all fine but one corner block, so that coarse and mixed rows are among them
+    box = [(0, 0, 0, n[0], n[1], 48), (0, 0, 48, n[0], 48, n[2]), (0, 48, 48, 48, n[1], n[2])]
+    sim, o = _pair(pf, n, dx, s, pos, vel, typ, boxes=box)
+    st = sim.step()
+    so, _ = o.step()
+    assert (st.active_cells, st.pinned_cell, st.iterations) == (so.active_cells, so.pinned_cell, so.iterations)
+    assert st.active_cells > 148 * 1024 * (2 if n[0] == 76 else 1)
+    assert abs(st.final_residual - so.final_residual) <= 1e-4 * so.final_residual
+    p, po = sim.cells()[1], o.cells()[1]
+    assert rel_err(p, po) < 1e-4, rel_err(p, po)
+    sim.close()
+
+
 def test_mr_face_shapes(pf):
     assert face_shape(5, 6, 7, 0) == (7, 6, 6)
