@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(PF_TV) k_fx_update(int nslots, SolveCtl* ctl, 
 // rc.ec over the coarse unknowns (grid-stride partials; the last CTA sums
 // them in order), then the guard and beta:
 //   r.z_j = flex[0], r.z_prev = flex[1], r.z_c = r.z_j + rc.ec
-constexpr int kGuardThreads = 256;
+constexpr int kGuardThreads = 256, kGuardBlocks = 64;
 
 __global__ void __launch_bounds__(kGuardThreads) k_fx_guard(SolveCtl* ctl, const float* rc, const float* ec, int nu,
                                                             int first, double min_gain, double* partials) {
@@ -306,10 +306,16 @@ __global__ void __launch_bounds__(kGuardThreads) k_fx_guard(SolveCtl* ctl, const
     am_last = atomicAdd(&ctl->counter, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!am_last || threadIdx.x != 0) return;
+  if (!am_last) return;
+  // the partials in order; all are loaded before the first addition (at most
+  // kGuardBlocks: a load per addition made this the longest part of the kernel)
   __threadfence();
+  __shared__ double part[kGuardBlocks];
+  if (threadIdx.x < gridDim.x) part[threadIdx.x] = __ldcg(&partials[kRedSlots * threadIdx.x]);
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   double D = 0.0;
-  for (int b = 0; b < (int)gridDim.x; ++b) D += __ldcg(&partials[kRedSlots * b]);
+  for (int b = 0; b < (int)gridDim.x; ++b) D += part[b];
   ctl->counter = 0;
   const double S1 = ctl->flex[0], Q = ctl->flex[1];
   const double S0 = S1 + D;
@@ -423,7 +429,7 @@ int coarse_solve(pf_ctx* ctx, int nslots, int precond) {
 int launch_guard(pf_ctx* ctx, bool coarse, int first, double min_gain) {
   CoarseOp& A = ((CoarseCtx*)ctx->learned)->op;
   const int nu = coarse ? 2 * A.nt : 0;
-  const int blocks = std::max(1, std::min((nu + kGuardThreads - 1) / kGuardThreads, 64));
+  const int blocks = std::max(1, std::min((nu + kGuardThreads - 1) / kGuardThreads, kGuardBlocks));
   ++ctx->launches;
   PF_CUDA_TRY(launch_pdl(k_fx_guard, dim3(blocks), dim3(kGuardThreads), ctx->stream, ctx->ctl, (const float*)A.rc,
                          (const float*)A.ec, nu, first, min_gain, ctx->partials));
