@@ -879,12 +879,34 @@ __global__ void __launch_bounds__(128) k_gconv(GConvArgs a) {
             make_uint2(pack_bf16(v[i].x, v[i].y), pack_bf16(v[i].z, v[i].w));
     }
   }
+  // Output geometry: lane (g, t) holds rows g (y = Y0 + 2yp) and g + 8 (y + 1),
+  // channels j*8 + 2t, +1.  The epilogue's operands are loaded here, so that
+  // their memory latency passes behind the products.
+  const int warp = tid >> 5, lane = tid & 31;
+  const int yp = warp & 1, wz = warp >> 1;
+  const int g = lane >> 2, t = lane & 3;
+  const int x = X0 + g, z = Z0 + wz;
+  bool inr[2];
+  int pos[2];
+  float2 gv[2][NT];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int y = Y0 + 2 * yp + h;
+    inr[h] = x < a.d.X && y < a.d.Y && z < a.d.Z;
+    pos[h] = x + a.d.X * (y + a.d.Y * z);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      gv[h][j] = make_float2(0.0f, 0.0f);
+      if (OUT == GOUT_GATE && inr[h])
+        gv[h][j] = __ldg(reinterpret_cast<const float2*>(a.gate + (size_t)pos[h] * kGS + j * 8 + 2 * t));
+      if (OUT == GOUT_SCALE && j == 0 && t == 0 && inr[h])
+        gv[h][0] = make_float2(inv_sqrt_diag(a.cop, pos[h], 0), inv_sqrt_diag(a.cop, pos[h], 1));
+    }
+  }
   asm volatile("cp.async.wait_all;\n" ::);
   __syncthreads();
 
   // 27 taps, A fragments prefetched kPre taps ahead, two accumulator sets (even / odd taps)
-  const int warp = tid >> 5, lane = tid & 31;
-  const int yp = warp & 1, wz = warp >> 1;
   const int lm = lane >> 3;
   const uint32_t abase = (uint32_t)__cvta_generic_to_shared(S) +
                          (uint32_t)(((lane & 7) + kGHX * (2 * yp + (lm & 1) + kGHY * wz)) * kGPitch + (lm >> 1) * 8) * 2;
@@ -909,29 +931,18 @@ __global__ void __launch_bounds__(128) k_gconv(GConvArgs a) {
     }
   }
 
-  // epilogue: lane (g, t) holds rows g (y = Y0 + 2yp) and g + 8 (y + 1), channels j*8 + 2t, +1
-  const int g = lane >> 2, t = lane & 3;
-  const int x = X0 + g, z = Z0 + wz;
   float r[NT][4];
 #pragma unroll
   for (int j = 0; j < NT; ++j)
 #pragma unroll
     for (int q = 0; q < 4; ++q) r[j][q] = acc[0][j][q] + acc[1][j][q];
-  bool inr[2];
-  int pos[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int y = Y0 + 2 * yp + h;
-    inr[h] = x < a.d.X && y < a.d.Y && z < a.d.Z;
-    pos[h] = x + a.d.X * (y + a.d.Y * z);
-  }
   if (OUT == GOUT_SCALE) {
     if (t == 0) {
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         if (inr[h])
           *reinterpret_cast<float2*>(a.y + (nb + pos[h]) * 2) =
-              make_float2(inv_sqrt_diag(a.cop, pos[h], 0) * r[0][2 * h], inv_sqrt_diag(a.cop, pos[h], 1) * r[0][2 * h + 1]);
+              make_float2(gv[h][0].x * r[0][2 * h], gv[h][0].y * r[0][2 * h + 1]);
     }
   } else if (OUT == GOUT_PLAIN) {
 #pragma unroll
@@ -950,8 +961,7 @@ __global__ void __launch_bounds__(128) k_gconv(GConvArgs a) {
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
         const int c0 = j * 8 + 2 * t;
-        const float2 gv = __ldg(reinterpret_cast<const float2*>(a.gate + (size_t)pos[h] * kGS + c0));
-        const float2 hv = make_float2(gv.x * r[j][2 * h], gv.y * r[j][2 * h + 1]);
+        const float2 hv = make_float2(gv[h][j].x * r[j][2 * h], gv[h][j].y * r[j][2 * h + 1]);
         *reinterpret_cast<float2*>(a.y + (nb + pos[h]) * kGS + c0) = hv;
         s[j].x += hv.x;
         s[j].y += hv.y;
