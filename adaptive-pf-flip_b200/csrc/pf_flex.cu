@@ -15,13 +15,14 @@
 //
 // Three fine-grid passes per iteration:
 //   spmv    Ap, p.Ap -> alpha
-//   update  x += alpha p, r -= alpha Ap, max|r|, r.D^-1 r, r.z_prev and the
-//           per-warp partial sums of the restriction rc = P^T r (z_prev is
-//           recomputed from the old r, so z is never stored)
+//   update  r -= alpha Ap, max|r|, r.D^-1 r, r.z_prev and the per-warp partial
+//           sums of the restriction rc = P^T r (z_prev is recomputed from the
+//           old r, so z is never stored)
 //   [coarse solve on the tile lattice: rc from the partials, ec = c(rc)]
 //   guard   r.P ec = rc.ec on the coarse lattice, so r.z_c = r.D^-1 r + rc.ec
 //           without another fine pass; accept or reject, beta
-//   dir     p = z + beta p
+//   dir     x += alpha p, p = z + beta p: x waits for the pass that loads p anyway
+//           (133 bytes a cell and iteration instead of 141)
 // The iteration body can be captured once into a CUDA graph and replayed.
 #include <algorithm>
 #include <cmath>
@@ -52,6 +53,7 @@ __global__ void k_fx_set(SolveCtl* ctl, double tol_abs, double tol_rel, int max_
   ctl->done = 0;
   ctl->it = 0;
   ctl->counter = 0;
+  ctl->e_pending = 0;
   ctl->aux[0] = 0.0;
   ctl->aux[2] = offered;
   if (reset) {
@@ -205,18 +207,22 @@ __global__ void __launch_bounds__(PF_TV, 4) k_fx_spmv(const int* __restrict__ nb
   const int l = threadIdx.x;
   double acc = 0.0;
   uint8_t kd_next = next_kind(kind, blockIdx.x, nslots, l);
+  int nb_next = nbr_lane(nbr, blockIdx.x, nslots);
   for (int s = blockIdx.x; s < nslots; s += gridDim.x) {
     const size_t o = (size_t)s * PF_TV + l;
     const uint8_t kd = kd_next;
+    const int nb = nb_next;
     kd_next = next_kind(kind, s + gridDim.x, nslots, l);
+    nb_next = nbr_lane(nbr, s + gridDim.x, nslots);
+    const int3 nt = neighbor_lanes(nb, l);
     if (!kd) continue;
     const V p0 = m.p[o];
     V ap;
     if (kd == 2) {
       ap = p0;
     } else {
-      long long no[6];
-      neighbor_offsets_tab(nbr, s, l, no);
+      int no[6];
+      neighbor_offsets_sel(nt, s, l, no);
       V off = (V)0;
       if (no[0] >= 0) off = fmav(m.cx[no[0]], m.p[no[0]], off);
       if (no[1] >= 0) off = fmav(m.cx[o], m.p[no[1]], off);
@@ -229,10 +235,10 @@ __global__ void __launch_bounds__(PF_TV, 4) k_fx_spmv(const int* __restrict__ nb
     m.Ap[o] = ap;
     acc = fmav((double)p0, (double)ap, acc);
   }
-  block_reduce_2(acc, 0.0, partials, ctl, kStagePAp);
+  block_reduce_1(acc, partials, ctl, kStagePAp);
 }
 
-// x/r update with max|r| (convergence), r.D^-1 r and r.z_prev of the new r,
+// r update with max|r| (convergence), r.D^-1 r and r.z_prev of the new r,
 // where z_prev = D^-1 r_old (+ P ec_old if the last direction used it); and
 // the warp partials of rc = P^T r_new when rc_part != nullptr
 template <typename V>
@@ -261,9 +267,8 @@ __global__ void __launch_bounds__(PF_TV) k_fx_update(int nslots, SolveCtl* ctl, 
     double rn = 0.0;
     if (kd) {
       const float ev = used_c && cl != 255 ? ec[coarse_index(tile, cl)] : 0.0f;
-      const V e = m.e[o], p = m.p[o], r_old = m.r[o], ap = m.Ap[o];
+      const V r_old = m.r[o], ap = m.Ap[o];
       const double di = inv_diag_at(m, kd, o);
-      m.e[o] = fmav(alpha, p, e);
       const V r = fmav(-alpha, ap, r_old);
       m.r[o] = r;
       rn = (double)r;
@@ -352,7 +357,8 @@ __global__ void __launch_bounds__(PF_TV) k_fx_dir(const int* slot_tile, int nslo
   pdl_wait();
   pdl_launch_dependents();
   if (ctl->done) return;
-  const V beta = (V)ctl->beta;
+  const V beta = (V)ctl->beta, alpha = (V)ctl->alpha;
+  const bool upd = ctl->e_pending != 0;
   const bool use_c = ctl->aux[0] != 0.0;
   const int l = threadIdx.x;
   uint8_t kd_next = next_kind(kind, blockIdx.x, nslots, l);
@@ -371,12 +377,26 @@ __global__ void __launch_bounds__(PF_TV) k_fx_dir(const int* slot_tile, int nslo
     if (!kd) continue;
     const float ev = use_c && cl != 255 ? ec[coarse_index(tile, cl)] : 0.0f;
     const double di = inv_diag_at(m, kd, o);
+    const V p = m.p[o], r = m.r[o], e = upd ? m.e[o] : (V)0;
     if (use_c) {
-      const double z = coarse_add((double)m.r[o], di, cl != 255 ? (double)ev : 0.0);
-      m.p[o] = fmav(beta, m.p[o], (V)z);
+      const double z = coarse_add((double)r, di, cl != 255 ? (double)ev : 0.0);
+      m.p[o] = fmav(beta, p, (V)z);
     } else {  // Jacobi only: one fma of r d^-1 over beta p
-      m.p[o] = (V)fmav((double)m.r[o], di, (double)(beta * m.p[o]));
+      m.p[o] = (V)fmav((double)r, di, (double)(beta * p));
     }
+    if (upd) m.e[o] = fmav(alpha, p, e);
+  }
+}
+
+// e += alpha p of the last update, when the solve ended before a direction pass
+template <typename V>
+__global__ void __launch_bounds__(PF_TV) k_fx_finish(int nslots, const SolveCtl* ctl, const uint8_t* kind,
+                                                     FlexVec<V> m) {
+  if (!ctl->e_pending) return;
+  const V alpha = (V)ctl->alpha;
+  for (int s = blockIdx.x; s < nslots; s += gridDim.x) {
+    const size_t o = (size_t)s * PF_TV + threadIdx.x;
+    if (kind[o]) m.e[o] = fmav(alpha, m.p[o], m.e[o]);
   }
 }
 
@@ -542,6 +562,8 @@ int flex_solve(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, FlexVec<V
     if (rc) return rc;
     if (check_every <= 0) batch = std::min(batch * 2, 64);
   }
+  (++ctx->launches), k_fx_finish<V><<<nred, PF_TV, 0, ctx->stream>>>(nslots, ctx->ctl, kind, m);
+  PF_CUDA_TRY(cudaGetLastError());
   *out = c;
   return PF_OK;
 }

@@ -132,6 +132,7 @@ struct SolveCtl {
   int min_fluid;
   int accepted, rejected;  // learned preconditioner outcomes
   double flex[2];          // flexible PCG: r.D^-1 r and r.z_prev of the current residual
+  int e_pending;           // flexible PCG: e lacks the last update's alpha p
 };
 
 constexpr int kMaxRedBlocks = 1184;  // 8 CTAs per SM on 148 SMs

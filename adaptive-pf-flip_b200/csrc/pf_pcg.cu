@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(PF_TV) k_spmv_plain(DevGrid G, int nslots, Sol
     v.Ap[o] = ap;
     acc = __dadd_rn(acc, __dmul_rn(p0, ap));
   }
-  block_reduce_2(acc, 0.0, partials, ctl, kStagePAp);
+  block_reduce_1(acc, partials, ctl, kStagePAp);
 }
 
 // Every pooled tile's six neighbour slots, nbr[6 s + d] in neighbor_slots'
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(PF_TV, 4) k_spmv_plain_tab(int nslots, SolveCt
     if (kd == 2) {
       ap = p0;
     } else {
-      long long no[6];
+      int no[6];
       neighbor_offsets_sel(nt, s, l, no);
       // +x -x +y -y +z -z, the reference's face order
       const double c[6] = {no[0] >= 0 ? v.cx[no[0]] : 0.0, v.cx[o], no[2] >= 0 ? v.cy[no[2]] : 0.0, v.cy[o],
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(PF_TV, 4) k_spmv_plain_tab(int nslots, SolveCt
     v.Ap[o] = ap;
     acc = __dadd_rn(acc, __dmul_rn(p0, ap));
   }
-  block_reduce_2(acc, 0.0, partials, ctl, kStagePAp);
+  block_reduce_1(acc, partials, ctl, kStagePAp);
 }
 
 __global__ void __launch_bounds__(PF_TV, 4) k_update_plain(int nslots, SolveCtl* ctl, const uint8_t* kind,
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(PF_TV) k_mixed_spmv(DevGrid G, int nslots, Sol
     m.Ap[o] = ap;
     acc += (double)p0 * (double)ap;
   }
-  block_reduce_2(acc, 0.0, partials, ctl, kStagePAp);
+  block_reduce_1(acc, partials, ctl, kStagePAp);
 }
 
 template <typename CC, typename CP>

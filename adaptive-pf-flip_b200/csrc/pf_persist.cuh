@@ -75,14 +75,6 @@ __device__ __forceinline__ bool ps_await(const PsPair* p, double& v, unsigned lo
 }
 __device__ __forceinline__ void ps_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
-// max of non-negative values over the warp, on every lane
-__device__ __forceinline__ double warp_max_nonneg(double v) {
-  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  return __hiloint2double((int)mh, (int)ml);
-}
-
 // Warp sums of N values at once (N a power of two up to 8), each by the tree
 // of warp_sum: at the first levels half of the lanes hand over one half of the
 // values and half the other, so N values take N + 4 - log2 N exchanges instead

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(PF_TV) k_assemble(DevGrid G, int nslots, Solve
     vec.r[o] = (V)rr;
     vec.x[o] = (V)0.0;
   }
-  block_reduce_2(rz, rmax, partials, ctl, /*stage=*/0, scale);
+  block_reduce_2(rz, rmax, partials, ctl, kStageInit);
 }
 
 }  // namespace

@@ -82,6 +82,7 @@ __device__ __forceinline__ void finalize_stage(SolveCtl* ctl, int stage, double 
     }
     case kStagePAp: {
       ctl->pAp = S;
+      ctl->e_pending = 0;  // the direction pass has run since the last update
       if (!isfinite(S)) ctl->done = 4;
       else if (fabs(S) < 1e-30 || !isfinite(ctl->rz / S)) ctl->done = 2;
       else ctl->alpha = ctl->rz / S;
@@ -127,6 +128,7 @@ __device__ __forceinline__ void finalize_stage(SolveCtl* ctl, int stage, double 
     }
     case kStageFlex: {
       ctl->it += 1;
+      ctl->e_pending = 1;
       ctl->res = M;
       ctl->flex[0] = S;
       ctl->flex[1] = S2;
@@ -138,19 +140,58 @@ __device__ __forceinline__ void finalize_stage(SolveCtl* ctl, int stage, double 
   }
 }
 
+// max of non-negative values over the warp, on every lane
+__device__ __forceinline__ double warp_max_nonneg(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+// Sum a, max b (non-negative; kMax) and sum c (kSum2) over the block in one
+// pass: the trees of block_sum_max with one exchange through shared memory
+// (result in thread 0).
+template <bool kMax, bool kSum2>
+__device__ __forceinline__ void block_fold(double& a, double& b, double& c, double (*sh)[32]) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    if (kSum2) c += __shfl_down_sync(0xffffffffu, c, o);
+  }
+  if (kMax) b = warp_max_nonneg(b);
+  if (lane == 0) {
+    sh[0][wid] = a;
+    if (kMax) sh[1][wid] = b;
+    if (kSum2) sh[2][wid] = c;
+  }
+  __syncthreads();
+  if (wid != 0) return;
+  a = lane < nw ? sh[0][lane] : 0.0;
+  if (kSum2) c = lane < nw ? sh[2][lane] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    if (kSum2) c += __shfl_down_sync(0xffffffffu, c, o);
+  }
+  if (kMax) b = warp_max_nonneg(lane < nw ? sh[1][lane] : 0.0);
+}
+
 // Per-CTA partial (sum a, max b, sum c) -> partials; the last CTA reduces all
 // partials in index order and finishes the stage.  Every CTA of the grid must
-// call this exactly once.
-__device__ __forceinline__ void block_reduce_3(double a, double b, double c, double* partials, SolveCtl* ctl,
-                                               int stage) {
+// call this exactly once.  Its latency ends every reducing pass, so the three
+// values share one pass of shuffles and barriers, and the last CTA loads all its
+// partials before it adds (0.5 us a pass less than value by value).
+template <bool kMax, bool kSum2>
+__device__ __forceinline__ void block_reduce(double a, double b, double c, double* partials, SolveCtl* ctl,
+                                             int stage) {
   __shared__ bool am_last;
-  double c2 = c, z0 = 0.0;
-  block_sum_max(a, b);
-  block_sum_max(c2, z0);
+  __shared__ double sh[2][3][32];
+  block_fold<kMax, kSum2>(a, b, c, sh[0]);
   if (threadIdx.x == 0) {
     partials[3 * blockIdx.x + 0] = a;
-    partials[3 * blockIdx.x + 1] = b;
-    partials[3 * blockIdx.x + 2] = c2;
+    if (kMax) partials[3 * blockIdx.x + 1] = b;
+    if (kSum2) partials[3 * blockIdx.x + 2] = c;
     __threadfence();
     const unsigned t = atomicAdd(&ctl->counter, 1u);
     am_last = (t == gridDim.x - 1);
@@ -158,24 +199,39 @@ __device__ __forceinline__ void block_reduce_3(double a, double b, double c, dou
   __syncthreads();
   if (!am_last) return;
   __threadfence();
-  double S = 0.0, M = 0.0, S2 = 0.0;
-  for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
-    S += __ldcg(&partials[3 * q + 0]);
-    M = fmax(M, __ldcg(&partials[3 * q + 1]));
-    S2 += __ldcg(&partials[3 * q + 2]);
+  constexpr int kPer = (kMaxRedBlocks + PF_TV - 1) / PF_TV;  // blocks of PF_TV threads
+  double v[kPer], m[kPer], w[kPer], S = 0.0, M = 0.0, S2 = 0.0;
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int q = threadIdx.x + u * blockDim.x;
+    const bool in = q < (int)gridDim.x;
+    v[u] = in ? __ldcg(&partials[3 * q + 0]) : 0.0;
+    m[u] = kMax && in ? __ldcg(&partials[3 * q + 1]) : 0.0;
+    w[u] = kSum2 && in ? __ldcg(&partials[3 * q + 2]) : 0.0;
   }
-  block_sum_max(S, M);
-  double z1 = 0.0;
-  block_sum_max(S2, z1);
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    if (threadIdx.x + u * blockDim.x >= gridDim.x) continue;
+    S += v[u];
+    M = fmax(M, m[u]);
+    S2 += w[u];
+  }
+  block_fold<kMax, kSum2>(S, M, S2, sh[1]);
   if (threadIdx.x == 0) {
-    finalize_stage(ctl, stage, S, M, S2);
+    finalize_stage(ctl, stage, S, M, kSum2 ? S2 : 0.0);
     ctl->counter = 0;
   }
 }
 
-__device__ __forceinline__ void block_reduce_2(double a, double b, double* partials, SolveCtl* ctl, int stage,
-                                               double /*unused*/ = 0.0) {
-  block_reduce_3(a, b, 0.0, partials, ctl, stage);
+__device__ __forceinline__ void block_reduce_3(double a, double b, double c, double* partials, SolveCtl* ctl,
+                                               int stage) {
+  block_reduce<true, true>(a, b, c, partials, ctl, stage);
+}
+__device__ __forceinline__ void block_reduce_2(double a, double b, double* partials, SolveCtl* ctl, int stage) {
+  block_reduce<true, false>(a, b, 0.0, partials, ctl, stage);
+}
+__device__ __forceinline__ void block_reduce_1(double a, double* partials, SolveCtl* ctl, int stage) {
+  block_reduce<false, false>(a, 0.0, 0.0, partials, ctl, stage);
 }
 
 // The streaming passes of the solvers walk their slots with a grid stride
@@ -254,16 +310,18 @@ __device__ __forceinline__ int3 neighbor_lanes(int nbl, int l) {
                    __shfl_sync(0xffffffffu, nbl, lz == 7 ? 4 : 5));
 }
 
-// neighbor_offsets_tab from the slots neighbor_lanes gave
-__device__ __forceinline__ void neighbor_offsets_sel(int3 t, int s, int l, long long* off) {
+// The six neighbours' offsets (order and meaning of neighbor_offsets) from the
+// slots neighbor_lanes gave, in 32 bits: the vectors of 2^31 cells would not fit
+// any device, and the 64-bit form costs the streaming passes registers.
+__device__ __forceinline__ void neighbor_offsets_sel(int3 t, int s, int l, int* off) {
   const int lx = l & 7, ly = (l >> 3) & 7, lz = l >> 6;
-  const long long base = (long long)s * PF_TV;
-  off[0] = lx < 7 ? base + l + 1 : (t.x >= 0 ? (long long)t.x * PF_TV + (l & ~7) : -1);
-  off[1] = lx > 0 ? base + l - 1 : (t.x >= 0 ? (long long)t.x * PF_TV + (l | 7) : -1);
-  off[2] = ly < 7 ? base + l + 8 : (t.y >= 0 ? (long long)t.y * PF_TV + (l & ~56) : -1);
-  off[3] = ly > 0 ? base + l - 8 : (t.y >= 0 ? (long long)t.y * PF_TV + (l | 56) : -1);
-  off[4] = lz < 7 ? base + l + 64 : (t.z >= 0 ? (long long)t.z * PF_TV + (l & ~448) : -1);
-  off[5] = lz > 0 ? base + l - 64 : (t.z >= 0 ? (long long)t.z * PF_TV + (l | 448) : -1);
+  const int base = s * PF_TV;
+  off[0] = lx < 7 ? base + l + 1 : (t.x >= 0 ? t.x * PF_TV + (l & ~7) : -1);
+  off[1] = lx > 0 ? base + l - 1 : (t.x >= 0 ? t.x * PF_TV + (l | 7) : -1);
+  off[2] = ly < 7 ? base + l + 8 : (t.y >= 0 ? t.y * PF_TV + (l & ~56) : -1);
+  off[3] = ly > 0 ? base + l - 8 : (t.y >= 0 ? t.y * PF_TV + (l | 56) : -1);
+  off[4] = lz < 7 ? base + l + 64 : (t.z >= 0 ? t.z * PF_TV + (l & ~448) : -1);
+  off[5] = lz > 0 ? base + l - 64 : (t.z >= 0 ? t.z * PF_TV + (l | 448) : -1);
 }
 
 // nbr[6 s + d] for every pooled slot (pf_flex.cu)
