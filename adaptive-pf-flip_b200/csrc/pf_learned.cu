@@ -314,9 +314,21 @@ int conv(pf_ctx* ctx, LearnedState* L, int layer, const float* x, int xs, const 
   const int bx = (d.X + kBrick - 1) / kBrick, by = (d.Y + kBrick - 1) / kBrick, bz = (d.Z + kBrick - 1) / kBrick;
   const int blocks = B * bx * by * bz;
   const int KC = xs / 16;
-  a.stage_w = brick_smem_w(KC, NT) <= kStageWeightsMax ? 1 : 0;
-  const size_t smem = (size_t)brick_smem_halo(KC) + (a.stage_w ? brick_smem_w(KC, NT) : 0);
+  // A lattice of few bricks gives every eight output channels a CTA of their
+  // own, with their weights staged: such a layer's time is the latency of one
+  // brick, 27 KC steps that each wait for NT weight loads from L2 otherwise (64
+  // to 64 channels on 5^3 tiles: 167 us).  The halo is staged once per slice, so
+  // large lattices keep one CTA per brick.
+  const bool sliced = NT > 1 && blocks * NT <= 4 * ctx->num_sms;
+  const int nts = sliced ? 1 : NT;
+  a.stage_w = sliced || brick_smem_w(KC, NT) <= kStageWeightsMax ? 1 : 0;
+  const size_t smem = (size_t)brick_smem_halo(KC) + (a.stage_w ? brick_smem_w(KC, nts) : 0);
   ++ctx->launches;
+  if (sliced) {
+    k_conv_brick<1><<<dim3(blocks, NT), 128, smem, ctx->stream>>>(a, bx, by, bz);
+    PF_CUDA_TRY(cudaGetLastError());
+    return PF_OK;
+  }
   switch (NT) {
     case 1: k_conv_brick<1><<<blocks, 128, smem, ctx->stream>>>(a, bx, by, bz); break;
     case 2: k_conv_brick<2><<<blocks, 128, smem, ctx->stream>>>(a, bx, by, bz); break;
@@ -334,7 +346,8 @@ int conv(pf_ctx* ctx, LearnedState* L, int layer, const float* x, int xs, const 
 // the widest input (128 channels) stages 58.75 KB, more than the default 48 KB
 int allow_brick_smem(pf_ctx* ctx) {
   const int bytes = brick_smem_halo(8) + kStageWeightsMax;
-  PF_CUDA_TRY(cudaFuncSetAttribute(k_conv_brick<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  PF_CUDA_TRY(cudaFuncSetAttribute(k_conv_brick<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   brick_smem_halo(8) + std::max(kStageWeightsMax, brick_smem_w(8, 1))));
   PF_CUDA_TRY(cudaFuncSetAttribute(k_conv_brick<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   PF_CUDA_TRY(cudaFuncSetAttribute(k_conv_brick<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   PF_CUDA_TRY(cudaFuncSetAttribute(k_conv_brick<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));

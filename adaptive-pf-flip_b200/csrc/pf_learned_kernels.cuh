@@ -149,10 +149,16 @@ __global__ void __launch_bounds__(128) k_conv_brick(ConvArgs a, int bx, int by, 
   const int b = brick / per_sample;
   brick -= b * per_sample;
   const int X0 = (brick % bx) * kBrick, Y0 = ((brick / bx) % by) * kBrick, Z0 = (brick / (bx * by)) * kBrick;
-  // small layers also stage their weight fragments (after the halo block)
-  const int nw = a.stage_w ? 27 * KC * NT * 32 : 0;
+  // this CTA's output tiles are j0 .. j0 + NT - 1 of ntot; staged weight
+  // fragments go after the halo block
+  const int j0 = blockIdx.y * NT, ntot = gridDim.y * NT;
+  const int nw = a.stage_w ? 27 * KC * NT * 16 : 0;  // uint4
   uint2* SW = reinterpret_cast<uint2*>(conv_smem + brick_smem_halo(KC));
-  for (int e = threadIdx.x; e < nw; e += blockDim.x) SW[e] = __ldg(a.wf + e);
+#pragma unroll 4
+  for (int e = threadIdx.x; e < nw; e += blockDim.x) {
+    const int step = e / (NT * 16), q = e - step * (NT * 16);
+    reinterpret_cast<uint4*>(SW)[e] = __ldg(reinterpret_cast<const uint4*>(a.wf) + (size_t)(step * ntot + j0) * 16 + q);
+  }
   // stage the halo block, two channels per item
   const int half = a.xs / 2;
 #pragma unroll 4
@@ -190,10 +196,11 @@ __global__ void __launch_bounds__(128) k_conv_brick(ConvArgs a, int bx, int by, 
       const uint32_t a1 = *reinterpret_cast<const uint32_t*>(r1 + kc * 16);
       const uint32_t a2 = *reinterpret_cast<const uint32_t*>(r0 + kc * 16 + 8);
       const uint32_t a3 = *reinterpret_cast<const uint32_t*>(r1 + kc * 16 + 8);
-      const size_t wo = ((size_t)(k * KC + kc) * NT) * 32 + lane;
+      const int ws = (k * KC + kc) * NT * 32 + lane;
+      const size_t wg = ((size_t)(k * KC + kc) * ntot + j0) * 32 + lane;
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
-        const uint2 bw = nw ? SW[wo + j * 32] : __ldg(a.wf + wo + j * 32);
+        const uint2 bw = nw ? SW[ws + j * 32] : __ldg(a.wf + wg + j * 32);
         mma_bf16(acc[j], a0, a1, a2, a3, bw.x, bw.y);
       }
     }
@@ -207,7 +214,7 @@ __global__ void __launch_bounds__(128) k_conv_brick(ConvArgs a, int bx, int by, 
     const float* gr = a.gmul ? a.gmul + (size_t)tpos * a.ys : nullptr;
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
-      const int c0 = j * 8 + 2 * t;
+      const int c0 = (j0 + j) * 8 + 2 * t;
       float o0 = acc[j][2 * h], o1 = acc[j][2 * h + 1];
       if (gr) {
         o0 *= gr[c0];
@@ -227,7 +234,8 @@ __global__ void __launch_bounds__(128) k_conv_brick(ConvArgs a, int bx, int by, 
       }
       *reinterpret_cast<float2*>(yr + c0) = make_float2(o0, o1);
     }
-    for (int c = NT * 8 + 2 * t; c < a.ys; c += 8) *reinterpret_cast<float2*>(yr + c) = make_float2(0.0f, 0.0f);
+    if (j0 + NT == ntot)
+      for (int c = ntot * 8 + 2 * t; c < a.ys; c += 8) *reinterpret_cast<float2*>(yr + c) = make_float2(0.0f, 0.0f);
   }
 }
 
