@@ -154,29 +154,37 @@ __global__ void __launch_bounds__(128) k_conv_brick(ConvArgs a, int bx, int by, 
   const int j0 = blockIdx.y * NT, ntot = gridDim.y * NT;
   const int nw = a.stage_w ? 27 * KC * NT * 16 : 0;  // uint4
   uint2* SW = reinterpret_cast<uint2*>(conv_smem + brick_smem_halo(KC));
-#pragma unroll 4
-  for (int e = threadIdx.x; e < nw; e += blockDim.x) {
-    const int step = e / (NT * 16), q = e - step * (NT * 16);
-    reinterpret_cast<uint4*>(SW)[e] = __ldg(reinterpret_cast<const uint4*>(a.wf) + (size_t)(step * ntot + j0) * 16 + q);
+  {
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(SW);
+    for (int e = threadIdx.x; e < nw; e += blockDim.x) {
+      const int step = e / (NT * 16), q = e - step * (NT * 16);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + e * 16),
+                   "l"(reinterpret_cast<const uint4*>(a.wf) + (size_t)(step * ntot + j0) * 16 + q));
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
   }
-  // stage the halo block, two channels per item
-  const int half = a.xs / 2;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < kHaloN * half; e += blockDim.x) {
-    const int hp = e / half, c2 = (e - hp * half) * 2;
+  // stage the halo block, four channels per item, the loads of eight items in
+  // flight (a load per item waited for memory 54 times a brick at 64 channels)
+  const int quarter = a.xs / 4;
+#pragma unroll 8
+  for (int e = threadIdx.x; e < kHaloN * quarter; e += blockDim.x) {
+    const int hp = e / quarter, c4 = (e - hp * quarter) * 4;
     const int x = X0 + hp % kHalo - 1, y = Y0 + (hp / kHalo) % kHalo - 1, z = Z0 + hp / (kHalo * kHalo) - 1;
-    float2 v = make_float2(0.0f, 0.0f);
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (x >= 0 && y >= 0 && z >= 0 && x < a.d.X && y < a.d.Y && z < a.d.Z) {
       const size_t q = (size_t)b * a.d.n + x + (size_t)a.d.X * (y + (size_t)a.d.Y * z);
-      v = *reinterpret_cast<const float2*>(a.x + q * a.xs + c2);
+      v = *reinterpret_cast<const float4*>(a.x + q * a.xs + c4);
       if (a.gate) {
-        const float2 gv = *reinterpret_cast<const float2*>(a.gate + q * a.xs + c2);
+        const float4 gv = *reinterpret_cast<const float4*>(a.gate + q * a.xs + c4);
         if (!(gv.x > 0.0f)) v.x = 0.0f;
         if (!(gv.y > 0.0f)) v.y = 0.0f;
+        if (!(gv.z > 0.0f)) v.z = 0.0f;
+        if (!(gv.w > 0.0f)) v.w = 0.0f;
       }
     }
-    *reinterpret_cast<uint32_t*>(S + (size_t)hp * pitch + c2) = pack_bf16(v.x, v.y);
+    *reinterpret_cast<uint2*>(S + (size_t)hp * pitch + c4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
   }
+  asm volatile("cp.async.wait_all;\n" ::);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
