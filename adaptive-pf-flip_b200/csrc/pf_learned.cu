@@ -169,13 +169,15 @@ LearnedState* get_state(pf_ctx* ctx, int* rc) {
 }
 
 int repack(pf_ctx* ctx, LearnedState* L) {
+  PackJobs J;
   for (int l = 0; l < kNumLayers; ++l) {
-    const int ci = kLayers[l].cin, co = kLayers[l].cout;
-    (++ctx->launches), k_pack<<<grid_for(frag_count(ci, co)), 256, 0, ctx->stream>>>(L->params + L->woff[l], ci, co,
-                                                                                      0, L->wf[l]);
-    (++ctx->launches), k_pack<<<grid_for(frag_count(co, ci)), 256, 0, ctx->stream>>>(L->params + L->woff[l], ci, co,
-                                                                                      1, L->wt[l]);
+    J.W[2 * l] = J.W[2 * l + 1] = L->params + L->woff[l];
+    J.out[2 * l] = L->wf[l];
+    J.out[2 * l + 1] = L->wt[l];
+    J.cin[l] = kLayers[l].cin;
+    J.cout[l] = kLayers[l].cout;
   }
+  (++ctx->launches), k_pack<<<dim3(32, 2 * kNumLayers), 256, 0, ctx->stream>>>(J);
   PF_CUDA_TRY(cudaGetLastError());
   return PF_OK;
 }

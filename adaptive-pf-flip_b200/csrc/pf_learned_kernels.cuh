@@ -73,7 +73,19 @@ __device__ __forceinline__ int neighbor(const Dims& d, int b, int x, int y, int 
 //   fwd: (tap, kc, nt, lane) -> {W[tap][kc*16+2t(+1)][nt*8+g], W[tap][kc*16+2t+8(+9)][nt*8+g]}
 //   bwd: the same for W'[tap][co][ci] = W[26 - tap][ci][co] (transposed, flipped)
 
-__global__ void k_pack(const float* W, int cin, int cout, int transpose, uint2* out) {
+// Every layer and direction in one launch (blockIdx.y): 32 launches of about 3 us
+// after every optimiser step otherwise.
+struct PackJobs {
+  const float* W[2 * kNumLayers];
+  uint2* out[2 * kNumLayers];
+  int cin[kNumLayers], cout[kNumLayers];
+};
+
+__global__ void k_pack(PackJobs J) {
+  const int layer = blockIdx.y >> 1, transpose = blockIdx.y & 1;
+  const float* W = J.W[blockIdx.y];
+  uint2* out = J.out[blockIdx.y];
+  const int cin = J.cin[layer], cout = J.cout[layer];
   const int ci_n = transpose ? cout : cin;   // GEMM K extent (input channels of this conv)
   const int co_n = transpose ? cin : cout;   // GEMM N extent
   const int KC = pad16(ci_n) / 16, NT = pad8(co_n) / 8;
