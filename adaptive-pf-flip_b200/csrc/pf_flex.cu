@@ -198,44 +198,88 @@ __global__ void k_build_nbr(DevGrid G, int nslots, int* nbr) {
   }
 }
 
+// p' Ap.  Bound by the bytes in flight: each cell waits for a dozen operands.  Two
+// cells per thread halve the load instructions and the address arithmetic and
+// let a warp keep twice the bytes in flight (256^3 cells: 192 -> 160 us a launch,
+// 49 bytes per cell at copy bandwidth are 125).  Four CTAs per SM: with three
+// and with five an iteration took 531 us instead of 497.  Taking the x
+// neighbours from the next lanes instead of from L1 changed nothing (164 us).
 template <typename V>
-__global__ void __launch_bounds__(PF_TV, 4) k_fx_spmv(const int* __restrict__ nbr, int nslots, SolveCtl* ctl,
-                                                   const uint8_t* kind, FlexVec<V> m, double* partials) {
+__global__ void __launch_bounds__(kPairNT, 4) k_fx_spmv(const int* __restrict__ nbr, int nslots, SolveCtl* ctl,
+                                                     const uint8_t* kind, FlexVec<V> m, double* partials) {
+  typedef typename PairOf<V>::type V2;
   pdl_wait();
   pdl_launch_dependents();
   if (ctl->done) return;
-  const int l = threadIdx.x;
-  double acc = 0.0;
-  uint8_t kd_next = next_kind(kind, blockIdx.x, nslots, l);
+  const int l = 2 * threadIdx.x;
+  const int lx = l & 7, ly = (l >> 3) & 7, lz = l >> 6;
+  double acc0 = 0.0, acc1 = 0.0;
+  auto kinds = [&](int s) {
+    return s < nslots ? *reinterpret_cast<const uchar2*>(kind + (size_t)s * PF_TV + l) : make_uchar2(0, 0);
+  };
+  uchar2 kd_next = kinds(blockIdx.x);
   int nb_next = nbr_lane(nbr, blockIdx.x, nslots);
   for (int s = blockIdx.x; s < nslots; s += gridDim.x) {
-    const size_t o = (size_t)s * PF_TV + l;
-    const uint8_t kd = kd_next;
+    const int o = s * PF_TV + l;
+    const uchar2 kd = kd_next;
     const int nb = nb_next;
-    kd_next = next_kind(kind, s + gridDim.x, nslots, l);
+    kd_next = kinds(s + gridDim.x);
     nb_next = nbr_lane(nbr, s + gridDim.x, nslots);
-    const int3 nt = neighbor_lanes(nb, l);
-    if (!kd) continue;
-    const V p0 = m.p[o];
-    V ap;
-    if (kd == 2) {
-      ap = p0;
-    } else {
-      int no[6];
-      neighbor_offsets_sel(nt, s, l, no);
-      V off = (V)0;
-      if (no[0] >= 0) off = fmav(m.cx[no[0]], m.p[no[0]], off);
-      if (no[1] >= 0) off = fmav(m.cx[o], m.p[no[1]], off);
-      if (no[2] >= 0) off = fmav(m.cy[no[2]], m.p[no[2]], off);
-      if (no[3] >= 0) off = fmav(m.cy[o], m.p[no[3]], off);
-      if (no[4] >= 0) off = fmav(m.cz[no[4]], m.p[no[4]], off);
-      if (no[5] >= 0) off = fmav(m.cz[o], m.p[no[5]], off);
-      ap = m.scale * fmav(m.d[o], p0, -off);
+    // the neighbour slot across the face this pair touches on each axis
+    const int tx = __shfl_sync(0xffffffffu, nb, lx == 6 ? 0 : 1), ty = __shfl_sync(0xffffffffu, nb, ly == 7 ? 2 : 3),
+              tz = __shfl_sync(0xffffffffu, nb, lz == 7 ? 4 : 5);
+    if (!kd.x && !kd.y) continue;
+    // offsets of the pair's neighbours (-1: that tile is not pooled)
+    const int xp = lx < 6 ? o + 2 : (tx >= 0 ? tx * PF_TV + (l & ~7) : -1);
+    const int xm = lx > 0 ? o - 1 : (tx >= 0 ? tx * PF_TV + (l | 7) : -1);
+    const int yp = ly < 7 ? o + 8 : (ty >= 0 ? ty * PF_TV + (l & ~56) : -1);
+    const int ym = ly > 0 ? o - 8 : (ty >= 0 ? ty * PF_TV + (l | 56) : -1);
+    const int zp = lz < 7 ? o + 64 : (tz >= 0 ? tz * PF_TV + (l & ~448) : -1);
+    const int zm = lz > 0 ? o - 64 : (tz >= 0 ? tz * PF_TV + (l | 448) : -1);
+    const V2 p = ld_pair(m.p + o), d = ld_pair(m.d + o);
+    const V2 cx = ld_pair(m.cx + o), cy = ld_pair(m.cy + o), cz = ld_pair(m.cz + o);
+    const V pxp = m.p[xp >= 0 ? xp : o], pxm = m.p[xm >= 0 ? xm : o], cxp = m.cx[xp >= 0 ? xp : o];
+    const V2 pyp = ld_pair(m.p + (yp >= 0 ? yp : o)), pym = ld_pair(m.p + (ym >= 0 ? ym : o)),
+             cyp = ld_pair(m.cy + (yp >= 0 ? yp : o));
+    const V2 pzp = ld_pair(m.p + (zp >= 0 ? zp : o)), pzm = ld_pair(m.p + (zm >= 0 ? zm : o)),
+             czp = ld_pair(m.cz + (zp >= 0 ? zp : o));
+    // each cell's terms in the order +x -x +y -y +z -z
+    V off0 = fmav(cx.y, p.y, (V)0), off1 = (V)0;
+    if (xm >= 0) off0 = fmav(cx.x, pxm, off0);
+    if (xp >= 0) off1 = fmav(cxp, pxp, off1);
+    off1 = fmav(cx.y, p.x, off1);
+    if (yp >= 0) {
+      off0 = fmav(cyp.x, pyp.x, off0);
+      off1 = fmav(cyp.y, pyp.y, off1);
     }
-    m.Ap[o] = ap;
-    acc = fmav((double)p0, (double)ap, acc);
+    if (ym >= 0) {
+      off0 = fmav(cy.x, pym.x, off0);
+      off1 = fmav(cy.y, pym.y, off1);
+    }
+    if (zp >= 0) {
+      off0 = fmav(czp.x, pzp.x, off0);
+      off1 = fmav(czp.y, pzp.y, off1);
+    }
+    if (zm >= 0) {
+      off0 = fmav(cz.x, pzm.x, off0);
+      off1 = fmav(cz.y, pzm.y, off1);
+    }
+    const V ap0 = kd.x == 2 ? p.x : m.scale * fmav(d.x, p.x, -off0);
+    const V ap1 = kd.y == 2 ? p.y : m.scale * fmav(d.y, p.y, -off1);
+    if (kd.x && kd.y) {
+      V2 ap;
+      ap.x = ap0;
+      ap.y = ap1;
+      *reinterpret_cast<V2*>(m.Ap + o) = ap;
+    } else if (kd.x) {
+      m.Ap[o] = ap0;
+    } else {
+      m.Ap[o + 1] = ap1;
+    }
+    if (kd.x) acc0 = fmav((double)p.x, (double)ap0, acc0);
+    if (kd.y) acc1 = fmav((double)p.y, (double)ap1, acc1);
   }
-  block_reduce_1(acc, partials, ctl, kStagePAp);
+  block_reduce_pairs(acc0, acc1, partials, ctl, kStagePAp);
 }
 
 // r update with max|r| (convergence), r.D^-1 r and r.z_prev of the new r,
@@ -467,7 +511,7 @@ int launch_iteration(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, con
   const bool coarse = precond != PF_PRECOND_JACOBI;
   const int* nbr = ((CoarseCtx*)ctx->learned)->nbr;
   ++ctx->launches;
-  PF_CUDA_TRY(launch_pdl(k_fx_spmv<V>, dim3(nred), dim3(PF_TV), ctx->stream, nbr, nslots, ctx->ctl, kind, m,
+  PF_CUDA_TRY(launch_pdl(k_fx_spmv<V>, dim3(nred), dim3(kPairNT), ctx->stream, nbr, nslots, ctx->ctl, kind, m,
                          ctx->partials));
   float* rc_part = coarse ? ((CoarseCtx*)ctx->learned)->rc_part : nullptr;
   ++ctx->launches;

@@ -234,6 +234,75 @@ __device__ __forceinline__ void block_reduce_1(double a, double* partials, Solve
   block_reduce<false, false>(a, 0.0, 0.0, partials, ctl, stage);
 }
 
+// ---- two cells per thread -------------------------------------------------
+// A pass over double2 (float2) pairs of x neighbours: kPairNT threads hold a
+// slot, thread j its cells 2j and 2j + 1.  Sixteen consecutive threads then hold
+// the 32 cells of one warp of the one-cell passes, and the sums below follow the
+// same trees.
+constexpr int kPairNT = PF_TV / 2;
+
+template <typename V> struct PairOf;
+template <> struct PairOf<double> { typedef double2 type; };
+template <> struct PairOf<float> { typedef float2 type; };
+template <typename V>
+__device__ __forceinline__ typename PairOf<V>::type ld_pair(const V* p) {
+  return *reinterpret_cast<const typename PairOf<V>::type*>(p);
+}
+
+// block_reduce_1 of a pass over pairs: a0 and a1 are the sums of the even and
+// the odd cells.
+__device__ __forceinline__ void block_reduce_pairs(double a0, double a1, double* partials, SolveCtl* ctl, int stage) {
+  __shared__ bool am_last;
+  __shared__ double sh[2][16];
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    a0 += __shfl_down_sync(0xffffffffu, a0, o, 16);
+    a1 += __shfl_down_sync(0xffffffffu, a1, o, 16);
+  }
+  if ((lane & 15) == 0) sh[0][threadIdx.x >> 4] = a0 + a1;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double v = lane < 16 ? sh[0][lane] : 0.0;
+    v = warp_sum(v);
+    if (lane == 0) {
+      partials[3 * blockIdx.x] = v;
+      __threadfence();
+      const unsigned t = atomicAdd(&ctl->counter, 1u);
+      am_last = (t == gridDim.x - 1);
+    }
+  }
+  __syncthreads();
+  if (!am_last) return;
+  __threadfence();
+  // as thread q of PF_TV sums partials q, q + PF_TV, ...: q = threadIdx.x and threadIdx.x + kPairNT
+  constexpr int kPer = (kMaxRedBlocks + PF_TV - 1) / PF_TV;
+  double v[2][kPer], S[2] = {0.0, 0.0};
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int q = threadIdx.x + h * kPairNT + u * PF_TV;
+      v[h][u] = q < (int)gridDim.x ? __ldcg(&partials[3 * q]) : 0.0;
+    }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if ((int)threadIdx.x + h * kPairNT + u * PF_TV < (int)gridDim.x) S[h] += v[h][u];
+    S[h] = warp_sum(S[h]);
+    if (lane == 0) sh[1][(threadIdx.x >> 5) + 8 * h] = S[h];
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double t = warp_sum(lane < 16 ? sh[1][lane] : 0.0);
+    if (lane == 0) {
+      finalize_stage(ctl, stage, t, 0.0, 0.0);
+      ctl->counter = 0;
+    }
+  }
+}
+
 // The streaming passes of the solvers walk their slots with a grid stride
 // and read each cell's kind before its operands.  They load the kind of the
 // next slot one trip ahead, so a trip waits for one round of memory latency
