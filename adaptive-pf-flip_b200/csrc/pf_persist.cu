@@ -291,7 +291,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
   }
   __syncthreads();
 
-  const int lx = l & 7, ly = (l >> 3) & 7, lz = l >> 6;
+  // Phase 1 gives a quarter of the CTA a slot and a thread two x neighbours: half
+  // the load instructions of one cell per thread, twice the bytes in flight.  Per
+  // iteration 88^3 cells 19.7 -> 16.7 us, 104^3 25.8 -> 22.4; 128^3 stays at 51,
+  // where an iteration moves 220 MB between L2 and the SMs and 100 MB to DRAM.
+  // Phase 2 and the direction lost by it (17.4, 23.0 and 53.3 us with all three).
+  const int quarter = threadIdx.x / kPairNT, l2 = 2 * (threadIdx.x % kPairNT);
+  const int px = l2 & 7, py = (l2 >> 3) & 7, pz = l2 >> 6;
   constexpr int N = kPsVirt / 2;  // a thread's virtual CTAs are half, half + 2, ...
   const int own = half + 2 * ps_owner<N>(lane);
   const bool writes = (lane & (32 / N - 1)) == 0 && own < nvirt;
@@ -329,47 +335,69 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
     arrivals += gridDim.x;
     alive = ps_barrier(A.bar, arrivals);
     if (!alive) break;
-    // ---- phase 1
-    double acc[N];
+    // ---- phase 1: two cells per thread, four slots at a time
+    {
+      double sum[2][2];  // [virtual CTA quarter + 4 v][even, odd cells]
 #pragma unroll
-    for (int u = 0; u < N; ++u) {
-      acc[u] = 0.0;
-      for (int m = half + 2 * u; m < k; m += kPsVirt) {
-        const int q = m * PF_TV + l, s = c + kPsGrid * m, o = s * PF_TV + l;
-        const uint8_t kd = s_kind[q];
-        if (!kd) continue;
-        const int* nb = s_nbr + 8 * m;
-        // the six neighbours, +x -x +y -y +z -z (the reference's face order); -1 where there is none
-        auto across = [&](int d, int cell) {
-          const int t = nb[d];
-          return t >= 0 ? t * PF_TV + cell : -1;
-        };
-        const int n[6] = {lx < 7 ? o + 1 : across(0, l & ~7),   lx > 0 ? o - 1 : across(1, l | 7),
-                          ly < 7 ? o + 8 : across(2, l & ~56),  ly > 0 ? o - 8 : across(3, l | 56),
-                          lz < 7 ? o + 64 : across(4, l & ~448), lz > 0 ? o - 64 : across(5, l | 448)};
-        const double dg = A.diag[o], p0 = P[o];
-        const double cf[6] = {n[0] >= 0 ? A.cx[n[0]] : 0.0, n[1] >= 0 ? A.cx[o] : 0.0,
-                              n[2] >= 0 ? A.cy[n[2]] : 0.0, n[3] >= 0 ? A.cy[o] : 0.0,
-                              n[4] >= 0 ? A.cz[n[4]] : 0.0, n[5] >= 0 ? A.cz[o] : 0.0};
-        double pn[6];
-#pragma unroll
-        for (int d = 0; d < 6; ++d) pn[d] = P[n[d] >= 0 ? n[d] : o];
-        double ap;
-        if (kd == 2) {
-          ap = p0;
-        } else {
-          double off = 0.0;
-#pragma unroll
-          for (int d = 0; d < 6; ++d)
-            if (cf[d] != 0.0) off = __dadd_rn(off, __dmul_rn(cf[d], pn[d]));
-          ap = __dmul_rn(A.scale, __dsub_rn(__dmul_rn(dg, p0), off));
+      for (int v = 0; v < 2; ++v) {
+        sum[v][0] = sum[v][1] = 0.0;
+        for (int m = quarter + 4 * v; m < k; m += kPsVirt) {
+          const int q = m * PF_TV + l2, s = c + kPsGrid * m, o = s * PF_TV + l2;
+          const uchar2 kd = *reinterpret_cast<const uchar2*>(s_kind + q);
+          if (!kd.x && !kd.y) continue;
+          const int* nb = s_nbr + 8 * m;
+          // the pair's neighbours; -1 where there is none
+          auto across = [&](int d, int cell) {
+            const int t = nb[d];
+            return t >= 0 ? t * PF_TV + cell : -1;
+          };
+          const int xp = px < 6 ? o + 2 : across(0, l2 & ~7), xm = px > 0 ? o - 1 : across(1, l2 | 7),
+                    yp = py < 7 ? o + 8 : across(2, l2 & ~56), ym = py > 0 ? o - 8 : across(3, l2 | 56),
+                    zp = pz < 7 ? o + 64 : across(4, l2 & ~448), zm = pz > 0 ? o - 64 : across(5, l2 | 448);
+          const double2 zero = make_double2(0.0, 0.0);
+          const double2 p = ld_pair(P + o), dg = ld_pair(A.diag + o), cx = ld_pair(A.cx + o);
+          const double2 cym = ym >= 0 ? ld_pair(A.cy + o) : zero, czm = zm >= 0 ? ld_pair(A.cz + o) : zero;
+          const double2 cyp = yp >= 0 ? ld_pair(A.cy + yp) : zero, czp = zp >= 0 ? ld_pair(A.cz + zp) : zero;
+          const double cxp = xp >= 0 ? A.cx[xp] : 0.0, cxm = xm >= 0 ? cx.x : 0.0;
+          const double pxp = P[xp >= 0 ? xp : o], pxm = P[xm >= 0 ? xm : o];
+          const double2 pyp = ld_pair(P + (yp >= 0 ? yp : o)), pym = ld_pair(P + (ym >= 0 ? ym : o));
+          const double2 pzp = ld_pair(P + (zp >= 0 ? zp : o)), pzm = ld_pair(P + (zm >= 0 ? zm : o));
+          double2 off = zero;  // each cell's faces in the reference's order, +x -x +y -y +z -z
+          auto face = [](double& sum, double cf, double pn) {
+            if (cf != 0.0) sum = __dadd_rn(sum, __dmul_rn(cf, pn));
+          };
+          face(off.x, cx.y, p.y);
+          face(off.y, cxp, pxp);
+          face(off.x, cxm, pxm);
+          face(off.y, cx.y, p.x);
+          face(off.x, cyp.x, pyp.x);
+          face(off.y, cyp.y, pyp.y);
+          face(off.x, cym.x, pym.x);
+          face(off.y, cym.y, pym.y);
+          face(off.x, czp.x, pzp.x);
+          face(off.y, czp.y, pzp.y);
+          face(off.x, czm.x, pzm.x);
+          face(off.y, czm.y, pzm.y);
+          double2 ap;
+          ap.x = kd.x == 2 ? p.x : __dmul_rn(A.scale, __dsub_rn(__dmul_rn(dg.x, p.x), off.x));
+          ap.y = kd.y == 2 ? p.y : __dmul_rn(A.scale, __dsub_rn(__dmul_rn(dg.y, p.y), off.y));
+          *reinterpret_cast<double2*>(s_za + q) = ap;
+          if (kd.x) sum[v][0] = __dadd_rn(sum[v][0], __dmul_rn(p.x, ap.x));
+          if (kd.y) sum[v][1] = __dadd_rn(sum[v][1], __dmul_rn(p.y, ap.y));
         }
-        s_za[q] = ap;
-        acc[u] = __dadd_rn(acc[u], __dmul_rn(p0, ap));
       }
+      // sixteen threads hold the 32 cells of a warp of phase 2; the same tree
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          sum[v][0] += __shfl_xor_sync(0xffffffffu, sum[v][0], w);
+          sum[v][1] += __shfl_xor_sync(0xffffffffu, sum[v][1], w);
+        }
+      if ((lane & 15) == 0)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) sh.loc[quarter + 4 * v][l2 >> 5] = sum[v][0] + sum[v][1];
     }
-    const double pap = warp_sum_many(acc);
-    if (writes) sh.loc[own][wid] = pap;
     double S = 0.0, M = 0.0;
     // No fence: the sums depend on every p read above, and the owners overwrite
     // p only with a value that depends on the sums.
@@ -380,7 +408,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
     sc.after_pap(S);
     if (sc.done) break;
     // ---- phase 2
-    double rmax = 0.0;
+    double acc[N], rmax = 0.0;
 #pragma unroll
     for (int u = 0; u < N; ++u) {
       acc[u] = 0.0;
