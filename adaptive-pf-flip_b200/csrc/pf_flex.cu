@@ -212,7 +212,6 @@ __global__ void __launch_bounds__(kPairNT, 4) k_fx_spmv(const int* __restrict__ 
   pdl_launch_dependents();
   if (ctl->done) return;
   const int l = 2 * threadIdx.x;
-  const int lx = l & 7, ly = (l >> 3) & 7, lz = l >> 6;
   double acc0 = 0.0, acc1 = 0.0;
   auto kinds = [&](int s) {
     return s < nslots ? *reinterpret_cast<const uchar2*>(kind + (size_t)s * PF_TV + l) : make_uchar2(0, 0);
@@ -225,17 +224,10 @@ __global__ void __launch_bounds__(kPairNT, 4) k_fx_spmv(const int* __restrict__ 
     const int nb = nb_next;
     kd_next = kinds(s + gridDim.x);
     nb_next = nbr_lane(nbr, s + gridDim.x, nslots);
-    // the neighbour slot across the face this pair touches on each axis
-    const int tx = __shfl_sync(0xffffffffu, nb, lx == 6 ? 0 : 1), ty = __shfl_sync(0xffffffffu, nb, ly == 7 ? 2 : 3),
-              tz = __shfl_sync(0xffffffffu, nb, lz == 7 ? 4 : 5);
+    int no[6];
+    neighbor_pairs(nb, s, l, no);
     if (!kd.x && !kd.y) continue;
-    // offsets of the pair's neighbours (-1: that tile is not pooled)
-    const int xp = lx < 6 ? o + 2 : (tx >= 0 ? tx * PF_TV + (l & ~7) : -1);
-    const int xm = lx > 0 ? o - 1 : (tx >= 0 ? tx * PF_TV + (l | 7) : -1);
-    const int yp = ly < 7 ? o + 8 : (ty >= 0 ? ty * PF_TV + (l & ~56) : -1);
-    const int ym = ly > 0 ? o - 8 : (ty >= 0 ? ty * PF_TV + (l | 56) : -1);
-    const int zp = lz < 7 ? o + 64 : (tz >= 0 ? tz * PF_TV + (l & ~448) : -1);
-    const int zm = lz > 0 ? o - 64 : (tz >= 0 ? tz * PF_TV + (l | 448) : -1);
+    const int xp = no[0], xm = no[1], yp = no[2], ym = no[3], zp = no[4], zm = no[5];
     const V2 p = ld_pair(m.p + o), d = ld_pair(m.d + o);
     const V2 cx = ld_pair(m.cx + o), cy = ld_pair(m.cy + o), cz = ld_pair(m.cz + o);
     const V pxp = m.p[xp >= 0 ? xp : o], pxm = m.p[xm >= 0 ? xm : o], cxp = m.cx[xp >= 0 ? xp : o];

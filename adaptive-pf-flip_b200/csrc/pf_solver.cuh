@@ -369,28 +369,23 @@ __device__ __forceinline__ int nbr_lane(const int* __restrict__ nbr, int s, int 
   return s < nslots && lane < 6 ? __ldg(nbr + 6 * (size_t)s + lane) : -1;
 }
 
-// The neighbour slot a cell needs per axis, from the entries nbr_lane gave:
-// the +side slot for a cell on the tile's high face, the -side slot
-// otherwise (only a cell on the low face uses it).  Every lane of the warp
-// must call it (shuffles).
-__device__ __forceinline__ int3 neighbor_lanes(int nbl, int l) {
+// The neighbours' offsets of the pair of cells l, l + 1 (l even) of slot s, order
+// and meaning of neighbor_offsets: +x of the second cell, -x of the first, the
+// first of the neighbouring pair for the other four.  nbl is what nbr_lane gave;
+// every lane of the warp must call it (shuffles).  In 32 bits: the vectors of
+// 2^31 cells would not fit any device, and 64 bits cost the passes registers.
+__device__ __forceinline__ void neighbor_pairs(int nbl, int s, int l, int (&off)[6]) {
   const int lx = l & 7, ly = (l >> 3) & 7, lz = l >> 6;
-  return make_int3(__shfl_sync(0xffffffffu, nbl, lx == 7 ? 0 : 1), __shfl_sync(0xffffffffu, nbl, ly == 7 ? 2 : 3),
-                   __shfl_sync(0xffffffffu, nbl, lz == 7 ? 4 : 5));
-}
-
-// The six neighbours' offsets (order and meaning of neighbor_offsets) from the
-// slots neighbor_lanes gave, in 32 bits: the vectors of 2^31 cells would not fit
-// any device, and the 64-bit form costs the streaming passes registers.
-__device__ __forceinline__ void neighbor_offsets_sel(int3 t, int s, int l, int* off) {
-  const int lx = l & 7, ly = (l >> 3) & 7, lz = l >> 6;
-  const int base = s * PF_TV;
-  off[0] = lx < 7 ? base + l + 1 : (t.x >= 0 ? t.x * PF_TV + (l & ~7) : -1);
-  off[1] = lx > 0 ? base + l - 1 : (t.x >= 0 ? t.x * PF_TV + (l | 7) : -1);
-  off[2] = ly < 7 ? base + l + 8 : (t.y >= 0 ? t.y * PF_TV + (l & ~56) : -1);
-  off[3] = ly > 0 ? base + l - 8 : (t.y >= 0 ? t.y * PF_TV + (l | 56) : -1);
-  off[4] = lz < 7 ? base + l + 64 : (t.z >= 0 ? t.z * PF_TV + (l & ~448) : -1);
-  off[5] = lz > 0 ? base + l - 64 : (t.z >= 0 ? t.z * PF_TV + (l | 448) : -1);
+  const int o = s * PF_TV + l;
+  // per axis, the slot across the one face of the tile that the pair can touch
+  const int tx = __shfl_sync(0xffffffffu, nbl, lx == 6 ? 0 : 1), ty = __shfl_sync(0xffffffffu, nbl, ly == 7 ? 2 : 3),
+            tz = __shfl_sync(0xffffffffu, nbl, lz == 7 ? 4 : 5);
+  off[0] = lx < 6 ? o + 2 : (tx >= 0 ? tx * PF_TV + (l & ~7) : -1);
+  off[1] = lx > 0 ? o - 1 : (tx >= 0 ? tx * PF_TV + (l | 7) : -1);
+  off[2] = ly < 7 ? o + 8 : (ty >= 0 ? ty * PF_TV + (l & ~56) : -1);
+  off[3] = ly > 0 ? o - 8 : (ty >= 0 ? ty * PF_TV + (l | 56) : -1);
+  off[4] = lz < 7 ? o + 64 : (tz >= 0 ? tz * PF_TV + (l & ~448) : -1);
+  off[5] = lz > 0 ? o - 64 : (tz >= 0 ? tz * PF_TV + (l | 448) : -1);
 }
 
 // nbr[6 s + d] for every pooled slot (pf_flex.cu)

@@ -1,4 +1,4 @@
-"""The PLAIN solve at every way its work is split over the GPU.
+"""The PLAIN solve at every way its work is split over the GPU, and the other modes beside it.
 
 A system's tiles go to 148 CTAs: one to eight tiles each live on chip (a kernel
 per count, 5 and 7 running in the next larger one's), more are streamed with as
@@ -21,7 +21,7 @@ from gpu_helpers import to_oracle_phase
 pytestmark = pytest.mark.gpu
 
 GRIDS = [(5, 6, 4), (39, 30, 22), (46, 47, 40), (54, 55, 62), (63, 62, 56), (64, 64, 64), (70, 71, 72), (78, 79, 72),
-         (80, 79, 77), (88, 86, 81), (104, 97, 90), (127, 118, 100)]
+         (80, 79, 77), (88, 86, 81), (104, 97, 90), (127, 118, 100), (160, 158, 155)]
 
 
 def _system(shape, seed, solids=True):
@@ -77,6 +77,28 @@ def test_mixed_reaches_the_plain_solution(pf, shape, bf16):
             g.set_field(f, v, np.ones(g.bdims(f)[::-1], np.uint8))
         st = pf.spProjectStepVC3D(g, pp, 1.0 / 60, 20000, 0.0, 0.01,
                                   solver=pf.SolverConfig(mode=mode, rel_tol=1e-9, bf16_storage=bf16))
+        assert st.converged and st.res_final < 1e-9 * st.res0
+        out.append(g.get_field(pf.PF_P)[0].astype(np.float64))
+        g.close()
+    assert np.abs(out[0] - out[1]).max() <= 1e-5 * np.abs(out[0]).max()
+
+
+@pytest.mark.parametrize("inner_fp32", [False, True])
+@pytest.mark.parametrize("shape", [(5, 6, 4), (39, 30, 22), (71, 57, 65), (96, 89, 82)], ids=str)
+def test_flexible_pcg_on_ragged_systems_reaches_the_plain_solution(pf, shape, inner_fp32):
+    """The flexible PCG takes the cells in pairs of x neighbours: pairs with one
+    fluid cell, pairs across tile and domain edges, one to several slots per
+    CTA.  Stop and tolerance as for the mixed mode above."""
+    fields = _system(shape, 2 + sum(shape), solids=False)
+    pp = pf.PhaseParams(1.0, 0.01)
+    out = []
+    for solver in (pf.SolverConfig(rel_tol=1e-9),
+                   pf.SolverConfig(mode=pf.PF_SOLVER_LEARNED, rel_tol=1e-9, precond=pf.PF_PRECOND_JACOBI,
+                                   inner_fp32=inner_fp32)):
+        g = pf.SparseMacGrid3D(*shape, 1.0 / max(shape), max_particles=int(np.prod(shape)) // 4 + 64)
+        for f, v in fields.items():
+            g.set_field(f, v, np.ones(g.bdims(f)[::-1], np.uint8))
+        st = pf.spProjectStepVC3D(g, pp, 1.0 / 60, 20000, 0.0, 0.01, solver=solver)
         assert st.converged and st.res_final < 1e-9 * st.res0
         out.append(g.get_field(pf.PF_P)[0].astype(np.float64))
         g.close()
