@@ -278,8 +278,7 @@ __global__ void __launch_bounds__(kPairNT, 4) k_fx_spmv(const int* __restrict__ 
 // where z_prev = D^-1 r_old (+ P ec_old if the last direction used it); and
 // the warp partials of rc = P^T r_new when rc_part != nullptr.  Four CTAs per
 // SM: unbounded it took 38 registers, three CTAs, and a third wave two thirds
-// full (256^3: 0.550 -> 0.529 ms per learned iteration; the SpMV at three or two
-// CTAs with more registers was slower, 0.584 and 0.635).
+// full (256^3: 0.550 -> 0.529 ms per learned iteration).
 template <typename V>
 __global__ void __launch_bounds__(PF_TV, 4) k_fx_update(int nslots, SolveCtl* ctl, const uint8_t* kind, FlexVec<V> m,
                                                      const int* slot_tile, const float* ec, float* rc_part,

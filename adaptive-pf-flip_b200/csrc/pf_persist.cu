@@ -7,7 +7,8 @@
 // three kernels of pf_pcg.cu.  Every operation rounds as there and the sums run
 // in the same order, so x, the iteration count and the residuals have the same
 // bits.  Per iteration, before (three launches) and now: 24^3 cells 21 -> 4.4 us,
-// 48^3 25 -> 5.6, 64^3 28.6 -> 7.7, 128^3 80 -> 51.
+// 48^3 25 -> 5.6, 64^3 28.6 -> 7.7, 128^3 80 -> 51.  Where the streaming kernel
+// ends, 148^3 takes 87 us and the three kernels at 152^3 101: 93 for as many cells.
 #include <algorithm>
 
 #include "pf_ctx.h"
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
   // Phase 1 gives a quarter of the CTA a slot and a thread two x neighbours: half
   // the load instructions of one cell per thread, twice the bytes in flight.  Per
   // iteration 88^3 cells 19.7 -> 16.7 us, 104^3 25.8 -> 22.4; 128^3 stays at 51,
-  // where an iteration moves 220 MB between L2 and the SMs and 100 MB to DRAM.
+  // where 220 MB per iteration pass through L2 and 100 MB of them to or from DRAM.
   // Phase 2 and the direction lost by it (17.4, 23.0 and 53.3 us with all three).
   const int quarter = threadIdx.x / kPairNT, l2 = 2 * (threadIdx.x % kPairNT);
   const int px = l2 & 7, py = (l2 >> 3) & 7, pz = l2 >> 6;
