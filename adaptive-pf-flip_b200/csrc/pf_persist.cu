@@ -478,12 +478,15 @@ cudaError_t launch_resident(const PsPlain& a, int k, int grid, cudaStream_t stre
   }
 }
 
+// `room` is what a CTA may take, whatever the system: the attribute belongs to
+// the kernel on this device, and another thread's context may be between setting
+// it and its launch.
 cudaError_t launch_stream(const PsPlain& a, int k, int grid, size_t room, cudaStream_t stream) {
   const size_t v = PF_TV * sizeof(double), base = k * ps_slot_bytes();
   int kr = (int)std::min<size_t>(k, (room - base) / v);
   int kx = (int)std::min<size_t>(k, (room - base - kr * v) / v);
   const size_t smem = base + (size_t)(kr + kx) * v;
-  const cudaError_t e = cudaFuncSetAttribute(k_plain_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = cudaFuncSetAttribute(k_plain_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<PsPlain*>(&a), &kr, &kx};
   return cudaLaunchCooperativeKernel((const void*)k_plain_stream, dim3(grid), dim3(kStreamThreads), args, smem,

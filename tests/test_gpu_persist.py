@@ -135,3 +135,38 @@ def test_launches_chain_bit_for_bit(pf):
     assert st.res_final == s2.res_final
     assert np.array_equal(g.get_field(pf.PF_P)[0], p.cpu().numpy())
     g.close()
+
+
+THREADS = """
+import threading
+import numpy as np
+from conftest import load_package
+from test_gpu_persist import _system
+pf = load_package()
+shapes, rounds, done = [(88, 86, 81), (127, 118, 100)], 20, {}
+
+def solve(g, shape):
+    for _ in range(rounds):
+        st = pf.spProjectStepVC3D(g, pf.PhaseParams(1.0, 0.01), 1.0 / 60, 1, 0.0, 0.01)
+        assert st.iterations == 1
+    done[shape] = True
+
+grids = []
+for s in shapes:
+    g = pf.SparseMacGrid3D(*s, 1.0 / max(s), max_particles=int(np.prod(s)) // 4 + 64)
+    for f, v in _system(s, sum(s)).items():
+        g.set_field(f, v, np.ones(g.bdims(f)[::-1], np.uint8))
+    grids.append(g)
+threads = [threading.Thread(target=solve, args=a) for a in zip(grids, shapes)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+assert len(done) == 2, "a thread's solve failed"
+"""
+
+
+def test_two_threads_solve_side_by_side(pf, tmp_path):
+    """Two contexts, a thread each, on systems whose streaming kernels take
+    different amounts of shared memory; every launch is held back for 3 ms after
+    it is set up, so one thread's set-up falls before the other's launch."""
+    from coop_shim import run_under_shim
+    run_under_shim(tmp_path, THREADS, delay_us=3000)
