@@ -1526,8 +1526,8 @@ int project_mr(pf_ctx* ctx, MrState* s, const pf_mr_step_cfg* cfg, pf_mr_step_st
   int launched = 0;
   stage_begin(ctx, PF_STAGE_PCG);
   const int rows = (N + kPsGrid * kMrResNT - 1) / (kPsGrid * kMrResNT);
-  const bool resident = rows <= kMrResRows && ctx->num_sms >= kPsGrid && cfg->cg_iters > 0;
-  if (resident) {
+  bool refused = false;
+  if (rows <= kMrResRows && ctx->num_sms >= kPsGrid && cfg->cg_iters > 0) {
     int* dead = s->counters + 8;
     // room for the slices: what the device gives a CTA less the static arrays
     const size_t smem = (ctx->smem_optin - sizeof(PsShared) - kMrResRows * (kMrResNT / 32) * sizeof(int) - 256) & ~(size_t)63;
@@ -1535,35 +1535,36 @@ int project_mr(pf_ctx* ctx, MrState* s, const pf_mr_step_cfg* cfg, pf_mr_step_st
     cap &= ~31;
     PF_CUDA_TRY(cudaMemsetAsync(dead, 0, sizeof(int), ctx->stream));
     PsBar bar{ctx->ps_entries, ctx->ps_counter};
-    for (int first = 1; !c.done && launched < cfg->cg_iters; first = 0) {
+    while (!c.done && launched < cfg->cg_iters) {
       unsigned long long tag = ctx->ps_tag + 1;
       ctx->ps_tag += 2 * kPsChunk;
-      PF_CUDA_TRY(cudaMemsetAsync(ctx->ps_counter, 0, sizeof(unsigned long long), ctx->stream));
-      int n = N, f = first;
+      int n = N, first = launched == 0;
       const int *sp = s->slice_ptr, *cl = s->col, *ar = tot + 3;
       const double* cf = s->coef;
-      void* args[] = {&n, &sp, &cl, &cf, &V, &s->ctl, &ar, &f, &bar, &tag, &dead, &cap};
+      void* args[] = {&n, &sp, &cl, &cf, &V, &s->ctl, &ar, &first, &bar, &tag, &dead, &cap};
       const void* kernel = rows == 1 ? (const void*)k_mr_pcg<1> : rows == 2 ? (const void*)k_mr_pcg<2>
                                                                             : (const void*)k_mr_pcg<3>;
-      PF_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      ++ctx->launches;
-      PF_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(kPsGrid), dim3(kMrResNT), args, smem, ctx->stream));
+      rc = ps_launch(ctx, kernel, kPsGrid, kMrResNT, args, smem, smem, &refused);
+      if (rc) return rc;
+      if (refused) break;
       PF_CUDA_TRY(cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(MrCtl), cudaMemcpyDeviceToHost, ctx->stream));
       PF_CUDA_TRY(cudaMemcpyAsync(s->h_ints + 4, dead, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
       if (s->h_ints[4]) return set_error(ctx, PF_ERR_CUDA, "multires pressure solve: a grid-wide wait ran out");
       c = *s->h_ctl;
-      launched += kPsChunk;
+      launched += std::min(kPsChunk, cfg->cg_iters - launched);
     }
   }
-  while (!resident) {
+  // the persistent kernel leaves its direction in pbuf[0], where these begin
+  const int before = launched;
+  while (refused || before == 0) {
     PF_CUDA_TRY(cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(MrCtl), cudaMemcpyDeviceToHost, ctx->stream));
     PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     c = *s->h_ctl;
     if (c.done || launched >= cfg->cg_iters) break;
     const int batch = std::min(kMrPoll, cfg->cg_iters - launched);
     for (int b = 0; b < batch; ++b) {
-      const int q = (launched + b) & 1;
+      const int q = (launched - before + b) & 1;
       double* p_prev = pbuf[q];
       double* p = pbuf[q ^ 1];
       // programmatic dependent launches: each kernel's CTAs are scheduled

@@ -371,15 +371,17 @@ int pcg_plain(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, PcgVec<dou
   if (nslots > 0)
     (++ctx->launches), k_plain_nbr<<<nblocks((size_t)6 * nslots, 256), 256, 0, ctx->stream>>>(G, nslots, ctx->nbr_plain);
   SolveCtl c{};
-  bool ran = false;
-  int rc = plain_persist(ctx, nslots, kind, ctx->nbr_plain, vec, scale, cfg->max_iter, &c, &ran);
-  if (!rc && !ran) rc = poll(ctx, &c);
+  int launched = 0;
+  int rc = plain_persist(ctx, nslots, kind, ctx->nbr_plain, vec, scale, cfg->max_iter, &c, &launched);
+  if (!rc && launched == 0) rc = poll(ctx, &c);
   if (rc) return rc;
   res->res0 = c.res0;
   res->tol = c.tol;
-  int launched = 0;
   int batch = cfg->check_every > 0 ? cfg->check_every : 4;
-  while (!ran && !c.done && launched < cfg->max_iter) {
+  // taken over from the persistent kernel: its iterations begin with the direction
+  if (launched > 0 && !c.done && launched < cfg->max_iter)
+    (++ctx->launches), k_direction_plain<<<nred, PF_TV, 0, ctx->stream>>>(nslots, ctx->ctl, kind, vec, scale);
+  while (!c.done && launched < cfg->max_iter) {
     const int nb = std::min(batch, cfg->max_iter - launched);
     for (int q = 0; q < nb; ++q) {
       (++ctx->launches), k_spmv_plain_tab<<<nred, kPairNT, 0, ctx->stream>>>(nslots, ctx->ctl, kind, ctx->nbr_plain, vec,
@@ -426,15 +428,17 @@ static int mixed_inner(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, M
   (++ctx->launches), k_mixed_start<CC, CP><<<nred, PF_TV, 0, ctx->stream>>>(nslots, ctx->ctl, kind, ctx->r, m, ctx->partials);
   PF_CUDA_TRY(cudaGetLastError());
   SolveCtl c{};
-  bool ran = false;
+  int launched = 0;
   const void* couplings[3] = {m.cx, m.cy, m.cz};
   int rc = mixed_persist(ctx, nslots, kind, ctx->nbr_plain, m.e, m.r, m.d, m.p, sizeof(CP) == 2, couplings,
-                         sizeof(CC) == 2, max_iter, &c, &ran);
-  if (!rc && !ran) rc = poll(ctx, &c);
+                         sizeof(CC) == 2, max_iter, &c, &launched);
+  if (!rc && launched == 0) rc = poll(ctx, &c);
   if (rc) return rc;
-  int launched = 0;
   int batch = check_every > 0 ? check_every : 4;
-  while (!ran && !c.done && launched < max_iter) {
+  // taken over from the persistent kernel: its iterations begin with the direction
+  if (launched > 0 && !c.done && launched < max_iter)
+    (++ctx->launches), k_mixed_direction<CC, CP><<<nred, PF_TV, 0, ctx->stream>>>(nslots, ctx->ctl, kind, m);
+  while (!c.done && launched < max_iter) {
     const int nb = std::min(batch, max_iter - launched);
     for (int q = 0; q < nb; ++q) {
       (++ctx->launches), k_mixed_spmv<CC, CP><<<nred, PF_TV, 0, ctx->stream>>>(G, nslots, ctx->ctl, kind, m, ctx->partials);

@@ -458,46 +458,54 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
 }
 
 template <int U>
-cudaError_t launch_resident(const PsPlain& a, int grid, cudaStream_t stream) {
+int launch_resident(pf_ctx* ctx, PsPlain& a, int grid, bool* refused) {
   const size_t smem = (size_t)U * kResSlotDoubles * sizeof(double);
-  const cudaError_t e =
-      cudaFuncSetAttribute(k_plain_resident<U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  void* args[] = {const_cast<PsPlain*>(&a)};
-  return cudaLaunchCooperativeKernel((const void*)k_plain_resident<U>, dim3(grid), dim3(PF_TV), args, smem, stream);
+  void* args[] = {&a};
+  return ps_launch(ctx, (const void*)k_plain_resident<U>, grid, PF_TV, args, smem, smem, refused);
 }
 
-cudaError_t launch_resident(const PsPlain& a, int k, int grid, cudaStream_t stream) {
+int launch_resident(pf_ctx* ctx, PsPlain& a, int k, int grid, bool* refused) {
   switch (k) {
-    case 1: return launch_resident<1>(a, grid, stream);
-    case 2: return launch_resident<2>(a, grid, stream);
-    case 3: return launch_resident<3>(a, grid, stream);
-    case 4: return launch_resident<4>(a, grid, stream);
-    case 5: case 6: return launch_resident<6>(a, grid, stream);
-    default: return launch_resident<8>(a, grid, stream);
+    case 1: return launch_resident<1>(ctx, a, grid, refused);
+    case 2: return launch_resident<2>(ctx, a, grid, refused);
+    case 3: return launch_resident<3>(ctx, a, grid, refused);
+    case 4: return launch_resident<4>(ctx, a, grid, refused);
+    case 5: case 6: return launch_resident<6>(ctx, a, grid, refused);
+    default: return launch_resident<8>(ctx, a, grid, refused);
   }
 }
 
-// `room` is what a CTA may take, whatever the system: the attribute belongs to
-// the kernel on this device, and another thread's context may be between setting
-// it and its launch.
-cudaError_t launch_stream(const PsPlain& a, int k, int grid, size_t room, cudaStream_t stream) {
+// room: what a CTA of this kernel may take
+int launch_stream(pf_ctx* ctx, PsPlain& a, int k, int grid, size_t room, bool* refused) {
   const size_t v = PF_TV * sizeof(double), base = k * ps_slot_bytes();
   int kr = (int)std::min<size_t>(k, (room - base) / v);
   int kx = (int)std::min<size_t>(k, (room - base - kr * v) / v);
-  const size_t smem = base + (size_t)(kr + kx) * v;
-  const cudaError_t e = cudaFuncSetAttribute(k_plain_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
-  if (e != cudaSuccess) return e;
-  void* args[] = {const_cast<PsPlain*>(&a), &kr, &kx};
-  return cudaLaunchCooperativeKernel((const void*)k_plain_stream, dim3(grid), dim3(kStreamThreads), args, smem,
-                                     stream);
+  void* args[] = {&a, &kr, &kx};
+  return ps_launch(ctx, (const void*)k_plain_stream, grid, kStreamThreads, args, room, base + (size_t)(kr + kx) * v,
+                   refused);
 }
 
 }  // namespace
 
+int ps_launch(pf_ctx* ctx, const void* kernel, int grid, int threads, void** args, size_t smem_max, size_t smem,
+              bool* refused) {
+  *refused = false;
+  PF_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
+  PF_CUDA_TRY(cudaMemsetAsync(ctx->ps_counter, 0, sizeof(unsigned long long), ctx->stream));
+  const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, ctx->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorLaunchOutOfResources) {
+    cudaGetLastError();  // not an error of the solve: leave none behind for the next check
+    *refused = true;
+    return PF_OK;
+  }
+  PF_CUDA_TRY(e);
+  ++ctx->launches;
+  return PF_OK;
+}
+
 int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, PcgVec<double> v, double scale,
-                  int max_iter, SolveCtl* out, bool* ran) {
-  *ran = false;
+                  int max_iter, SolveCtl* out, int* launched) {
+  *launched = 0;
   if (nslots <= 0 || ctx->num_sms < kPsGrid) return PF_OK;
   const int grid = std::min(nslots, kPsGrid), k = (nslots + kPsGrid - 1) / kPsGrid;
   const size_t room = ctx->smem_optin - sizeof(PsShared) - 64;
@@ -505,17 +513,17 @@ int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
   if (!resident && k * ps_slot_bytes() > room) return PF_OK;
   PsPlain a{nslots, std::min(nslots, kMaxRedBlocks), ctx->ctl, kind, nbr, v.x, v.r, v.p, v.z, v.diag, v.cx, v.cy,
             v.cz, scale, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0};
-  *ran = max_iter > 0;
-  for (int launched = 0; !out->done && launched < max_iter; launched += kPsChunk) {
+  while (!out->done && *launched < max_iter) {
     a.tag = ctx->ps_tag + 1;
     ctx->ps_tag += kPsChunk;
-    PF_CUDA_TRY(cudaMemsetAsync(ctx->ps_counter, 0, sizeof(unsigned long long), ctx->stream));
-    ++ctx->launches;
-    PF_CUDA_TRY(resident ? launch_resident(a, k, grid, ctx->stream) : launch_stream(a, k, grid, room, ctx->stream));
+    bool refused = false;
+    const int rc = resident ? launch_resident(ctx, a, k, grid, &refused) : launch_stream(ctx, a, k, grid, room, &refused);
+    if (rc || refused) return rc;
     PF_CUDA_TRY(cudaMemcpyAsync(ctx->h_ctl, ctx->ctl, sizeof(SolveCtl), cudaMemcpyDeviceToHost, ctx->stream));
     PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     *out = *ctx->h_ctl;
     if (out->aux[0] != 0.0) return set_error(ctx, PF_ERR_CUDA, "pressure solve: a grid-wide wait ran out");
+    *launched += std::min(kPsChunk, max_iter - *launched);
   }
   return PF_OK;
 }

@@ -220,47 +220,45 @@ __global__ void __launch_bounds__(PF_TV, 1) k_mixed_resident(PsMixed A) {
 }
 
 template <int U>
-cudaError_t launch_mixed(const PsMixed& a, int grid, cudaStream_t stream) {
+int launch_mixed(pf_ctx* ctx, PsMixed& a, int grid, bool* refused) {
   const size_t smem = (size_t)U * kMixSlotFloats * sizeof(float);
-  const cudaError_t e =
-      cudaFuncSetAttribute(k_mixed_resident<U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  void* args[] = {const_cast<PsMixed*>(&a)};
-  return cudaLaunchCooperativeKernel((const void*)k_mixed_resident<U>, dim3(grid), dim3(PF_TV), args, smem, stream);
+  void* args[] = {&a};
+  return ps_launch(ctx, (const void*)k_mixed_resident<U>, grid, PF_TV, args, smem, smem, refused);
+}
+
+int launch_mixed(pf_ctx* ctx, PsMixed& a, int k, int grid, bool* refused) {
+  switch (k) {
+    case 1: return launch_mixed<1>(ctx, a, grid, refused);
+    case 2: return launch_mixed<2>(ctx, a, grid, refused);
+    case 3: return launch_mixed<3>(ctx, a, grid, refused);
+    case 4: return launch_mixed<4>(ctx, a, grid, refused);
+    case 5: case 6: return launch_mixed<6>(ctx, a, grid, refused);
+    default: return launch_mixed<8>(ctx, a, grid, refused);
+  }
 }
 
 }  // namespace
 
 int mixed_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, float* e, float* r, const float* d,
-                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, SolveCtl* out, bool* ran) {
+                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, SolveCtl* out, int* launched) {
   const int k = (nslots + kPsGrid - 1) / kPsGrid, grid = std::min(nslots, kPsGrid);
-  *ran = nslots > 0 && ctx->num_sms >= kPsGrid && k <= kPsVirt;
-  if (!*ran) return PF_OK;
+  *launched = 0;
+  if (nslots <= 0 || ctx->num_sms < kPsGrid || k > kPsVirt) return PF_OK;
   PsMixed a{nslots, std::min(nslots, kMaxRedBlocks), 1, cc16, cp16, ctx->ctl, kind, nbr, e, r, d, p,
             {c[0], c[1], c[2]}, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0};
-  int launched = 0;
-  do {
+  while (!out->done && *launched < max_iter) {
     a.tag = ctx->ps_tag + 1;
     ctx->ps_tag += kPsChunk;
-    PF_CUDA_TRY(cudaMemsetAsync(ctx->ps_counter, 0, sizeof(unsigned long long), ctx->stream));
-    ++ctx->launches;
-    cudaError_t le = cudaSuccess;
-    switch (k) {
-      case 1: le = launch_mixed<1>(a, grid, ctx->stream); break;
-      case 2: le = launch_mixed<2>(a, grid, ctx->stream); break;
-      case 3: le = launch_mixed<3>(a, grid, ctx->stream); break;
-      case 4: le = launch_mixed<4>(a, grid, ctx->stream); break;
-      case 5: case 6: le = launch_mixed<6>(a, grid, ctx->stream); break;
-      default: le = launch_mixed<8>(a, grid, ctx->stream); break;
-    }
-    PF_CUDA_TRY(le);
+    bool refused = false;
+    const int rc = launch_mixed(ctx, a, k, grid, &refused);
+    if (rc || refused) return rc;
     PF_CUDA_TRY(cudaMemcpyAsync(ctx->h_ctl, ctx->ctl, sizeof(SolveCtl), cudaMemcpyDeviceToHost, ctx->stream));
     PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     *out = *ctx->h_ctl;
     if (out->aux[0] != 0.0) return set_error(ctx, PF_ERR_CUDA, "pressure solve: a grid-wide wait ran out");
     a.first = 0;
-    launched += kPsChunk;
-  } while (!out->done && launched < max_iter);
+    *launched += std::min(kPsChunk, max_iter - *launched);
+  }
   return PF_OK;
 }
 

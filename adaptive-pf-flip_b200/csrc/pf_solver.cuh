@@ -410,14 +410,26 @@ int solve_inner_outer(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, co
 // solver drivers (pf_pcg.cu)
 int pcg_plain(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, PcgVec<double> vec, double scale,
               const pf_solve_cfg* cfg, SolveResult* res);
-// PLAIN as a persistent kernel (pf_persist.cu); *ran is false when the system
-// has too many slots for it, and nothing was done
+// PLAIN as a persistent kernel (pf_persist.cu).  *launched: the iterations it was
+// launched for, 0 when the system has too many slots for it or the device refuses
+// its first launch (nothing was done then).  When it returns PF_OK with neither
+// out->done nor max_iter reached, a later launch was refused: the vectors and the
+// control block are those after an update, and the next pass is the direction.
 int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, PcgVec<double> v, double scale,
-                  int max_iter, SolveCtl* out, bool* ran);
+                  int max_iter, SolveCtl* out, int* launched);
 // MIXED's inner solve (started by k_mixed_start) as a persistent kernel
-// (pf_persist_mixed.cu); *ran as above
+// (pf_persist_mixed.cu); *launched as above
 int mixed_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, float* e, float* r, const float* d,
-                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, SolveCtl* out, bool* ran);
+                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, SolveCtl* out, int* launched);
+// One cooperative launch of a persistent kernel, its arrival counter cleared before.
+// *refused: the device has no place for all its CTAs at once (a part of the GPU is
+// set aside for another process, for one) or launches nothing cooperatively;
+// nothing has run then, and the caller's other kernels do the work.  smem_max, the
+// most this kernel may ask for, must not depend on the system: the attribute it
+// sets is the kernel's on this device, and another thread's context may be between
+// setting it and its launch.
+int ps_launch(pf_ctx* ctx, const void* kernel, int grid, int threads, void** args, size_t smem_max, size_t smem,
+              bool* refused);
 int solve_mixed(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, double scale, const pf_solve_cfg* cfg,
                 const void* phase_consts, SolveResult* res);
 int ensure_solver_buffers(pf_ctx* ctx, int mode);

@@ -170,3 +170,55 @@ def test_two_threads_solve_side_by_side(pf, tmp_path):
     it is set up, so one thread's set-up falls before the other's launch."""
     from coop_shim import run_under_shim
     run_under_shim(tmp_path, THREADS, delay_us=3000)
+
+
+# one slot a CTA, five and seven in the next larger kernels, eight, streaming with
+# r and x kept and with part of them kept
+BITS = [((39, 30, 22), (0, 1, 2)), ((70, 71, 72), (0, 2)), ((78, 79, 72), ()), ((80, 79, 77), (0, 1, 2)),
+        ((88, 86, 81), ()), ((127, 118, 100), ())]
+
+
+def solve_all(pf, check_every=0, its=23):
+    """A few iterations of PLAIN on every system and of MIXED where the second
+    entry names its storage modes; all outputs."""
+    out = {}
+    for shape, bf16 in BITS:
+        g = pf.SparseMacGrid3D(*shape, 1.0 / max(shape), max_particles=int(np.prod(shape)) // 4 + 64)
+        fields = _system(shape, 3 + sum(shape), solids=False)
+        cases = [("plain", pf.SolverConfig(check_every=check_every), its)]
+        cases += [(f"mixed{b}", pf.SolverConfig(mode=pf.PF_SOLVER_MIXED, bf16_storage=b, check_every=check_every,
+                                                rel_tol=1e-7), 300) for b in bf16]
+        for name, solver, n in cases:
+            for f, v in fields.items():
+                g.set_field(f, v, np.ones(g.bdims(f)[::-1], np.uint8))
+            st = pf.spProjectStepVC3D(g, pf.PhaseParams(1.0, 0.01), 1.0 / 60, n, 0.0, 0.01, solver=solver)
+            key = f"{shape}_{name}"
+            out[key] = g.get_field(pf.PF_P)[0]
+            out[key + "_stats"] = np.array([st.iterations, st.refinements, st.converged, st.breakdown, st.res_final])
+        g.close()
+    return out
+
+
+SOLVE_ALL = """
+import sys
+import numpy as np
+from conftest import load_package
+from test_gpu_persist import solve_all
+np.savez({path!r}, **solve_all(load_package(), {check_every}))
+"""
+
+
+def _same_bits(a, b):
+    assert sorted(a) == sorted(b)
+    for k in a:
+        assert np.array_equal(a[k], b[k], equal_nan=True), k
+
+
+def test_refused_launches_leave_the_work_to_the_kernels_per_iteration(pf, tmp_path):
+    """A device that refuses the cooperative launches (the shim answers them as one
+    without room for the grid does) solves by the kernels per iteration: the same
+    bits, PLAIN at every way its slots are kept and MIXED in its three storages."""
+    from coop_shim import run_under_shim
+    path = str(tmp_path / "refused.npz")
+    run_under_shim(tmp_path, SOLVE_ALL.format(path=path, check_every=0), allow=0)
+    _same_bits(solve_all(pf), dict(np.load(path)))
