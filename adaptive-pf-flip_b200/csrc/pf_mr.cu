@@ -852,7 +852,7 @@ template <int R>
 __global__ void __launch_bounds__(kMrResNT, 1) k_mr_pcg(int N, const int* __restrict__ slice_ptr,
                                                       const int* __restrict__ col, const double* __restrict__ coef,
                                                       MrVecs V, MrCtl* ctl_g, const int* air, int first, PsBar bar,
-                                                      unsigned long long tag0, int* dead, int cap) {
+                                                      unsigned long long tag0, int turns, int* dead, int cap) {
   extern __shared__ double s_coef[];  // [cap], then the columns [cap]
   __shared__ PsShared sh;
   __shared__ int s_at[R * (kMrResNT / 32)];  // each slice's length, then its place (-1: not kept)
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(kMrResNT, 1) k_mr_pcg(int N, const int* __rest
     return ps_wait<kMax>(sh, bar, which, parity, tag, kPsGrid * (kMrResNT / PF_TV), arrivals, S, M,
                          [] { return true; });
   };
-  for (int turn = 0; turn < kPsChunk && !ctl.done; ++turn) {
+  for (int turn = 0; turn < turns && !ctl.done; ++turn) {
     const int par = turn & 1;
     const unsigned long long tag = tag0 + 2 * turn;
 #pragma unroll
@@ -1537,11 +1537,12 @@ int project_mr(pf_ctx* ctx, MrState* s, const pf_mr_step_cfg* cfg, pf_mr_step_st
     PsBar bar{ctx->ps_entries, ctx->ps_counter};
     while (!c.done && launched < cfg->cg_iters) {
       unsigned long long tag = ctx->ps_tag + 1;
-      ctx->ps_tag += 2 * kPsChunk;
+      int turns = std::min(kPsTurns, cfg->cg_iters - launched);
+      ctx->ps_tag += 2 * turns;
       int n = N, first = launched == 0;
       const int *sp = s->slice_ptr, *cl = s->col, *ar = tot + 3;
       const double* cf = s->coef;
-      void* args[] = {&n, &sp, &cl, &cf, &V, &s->ctl, &ar, &first, &bar, &tag, &dead, &cap};
+      void* args[] = {&n, &sp, &cl, &cf, &V, &s->ctl, &ar, &first, &bar, &tag, &turns, &dead, &cap};
       const void* kernel = rows == 1 ? (const void*)k_mr_pcg<1> : rows == 2 ? (const void*)k_mr_pcg<2>
                                                                             : (const void*)k_mr_pcg<3>;
       rc = ps_launch(ctx, kernel, kPsGrid, kMrResNT, args, smem, smem, &refused);
@@ -1552,7 +1553,7 @@ int project_mr(pf_ctx* ctx, MrState* s, const pf_mr_step_cfg* cfg, pf_mr_step_st
       PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
       if (s->h_ints[4]) return set_error(ctx, PF_ERR_CUDA, "multires pressure solve: a grid-wide wait ran out");
       c = *s->h_ctl;
-      launched += std::min(kPsChunk, cfg->cg_iters - launched);
+      launched += turns;
     }
   }
   // the persistent kernel leaves its direction in pbuf[0], where these begin

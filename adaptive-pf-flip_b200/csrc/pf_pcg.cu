@@ -372,7 +372,7 @@ int pcg_plain(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, PcgVec<dou
     (++ctx->launches), k_plain_nbr<<<nblocks((size_t)6 * nslots, 256), 256, 0, ctx->stream>>>(G, nslots, ctx->nbr_plain);
   SolveCtl c{};
   int launched = 0;
-  int rc = plain_persist(ctx, nslots, kind, ctx->nbr_plain, vec, scale, cfg->max_iter, &c, &launched);
+  int rc = plain_persist(ctx, nslots, kind, ctx->nbr_plain, vec, scale, cfg->max_iter, cfg->check_every, &c, &launched);
   if (!rc && launched == 0) rc = poll(ctx, &c);
   if (rc) return rc;
   res->res0 = c.res0;
@@ -431,10 +431,11 @@ static int mixed_inner(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, M
   int launched = 0;
   const void* couplings[3] = {m.cx, m.cy, m.cz};
   int rc = mixed_persist(ctx, nslots, kind, ctx->nbr_plain, m.e, m.r, m.d, m.p, sizeof(CP) == 2, couplings,
-                         sizeof(CC) == 2, max_iter, &c, &launched);
+                         sizeof(CC) == 2, max_iter, check_every, &c, &launched);
   if (!rc && launched == 0) rc = poll(ctx, &c);
   if (rc) return rc;
-  int batch = check_every > 0 ? check_every : 4;
+  // one poll in the middle of the budget, one at its end
+  const int batch = check_every > 0 ? check_every : std::max(1, max_iter / 2);
   // taken over from the persistent kernel: its iterations begin with the direction
   if (launched > 0 && !c.done && launched < max_iter)
     (++ctx->launches), k_mixed_direction<CC, CP><<<nred, PF_TV, 0, ctx->stream>>>(nslots, ctx->ctl, kind, m);
@@ -449,7 +450,6 @@ static int mixed_inner(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, M
     launched += nb;
     rc = poll(ctx, &c);
     if (rc) return rc;
-    if (check_every <= 0) batch = std::min(batch * 2, 64);
   }
   *iters += c.it;
   *out = c;
@@ -465,10 +465,8 @@ struct MixedInner final : InnerSolver {
   MixVec<CC, CP> m{};
   int solve(pf_ctx* ctx, double eta, int max_iter, bool, const float** z, int* iters) override {
     SolveCtl ic{};
-    // one poll in the middle of the budget, one at its end
-    const int poll_at = check_every > 0 ? check_every : std::max(1, max_iter / 2);
     int before = 0;
-    const int rc = mixed_inner<CC, CP>(ctx, nslots, nred, kind, m, 0.0, eta, max_iter, poll_at, &before, &ic);
+    const int rc = mixed_inner<CC, CP>(ctx, nslots, nred, kind, m, 0.0, eta, max_iter, check_every, &before, &ic);
     if (rc) return rc;
     *iters = ic.it;
     *z = m.e;

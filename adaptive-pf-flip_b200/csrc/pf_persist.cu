@@ -28,6 +28,7 @@ struct PsPlain {
   PsBar bar;
   PsPair* faces;  // [2][nslots][6][64]
   unsigned long long tag;
+  int turns;      // iterations of this launch, at most
 };
 
 // r / d, correctly rounded, from inv = RN(1 / d) formed once per solve: the
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(PF_TV, 1) k_plain_resident(PsPlain A) {
   const bool writes = (lane & (32 / N - 1)) == 0;
   bool alive = true;
   unsigned long long arrivals = 0;
-  for (int turn = 0; turn < kPsChunk && !sc.done; ++turn) {
+  for (int turn = 0; turn < A.turns && !sc.done; ++turn) {
     const int par = turn & 1;
     const unsigned long long tag = A.tag + turn;
     // ---- phase 1
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
   const bool writes = (lane & (32 / N - 1)) == 0 && own < nvirt;
   bool pend = false, alive = true;
   unsigned long long arrivals = 0;
-  for (int turn = 0; turn < kPsChunk && !sc.done; ++turn) {
+  for (int turn = 0; turn < A.turns && !sc.done; ++turn) {
     const int par = turn & 1;
     const unsigned long long tag = A.tag + turn;
     // ---- direction
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
     pend = true;
     sc.after_update(S, M);
   }
-  // x's last update, and the state of the next launch when the chunk is over
+  // x's last update, and the state of the next launch when this one's turns are over
   for (int m = half; m < k; m += 2) {
     const int q = m * PF_TV + l;
     const size_t o = (size_t)(c + kPsGrid * m) * PF_TV + l;
@@ -504,7 +505,7 @@ int ps_launch(pf_ctx* ctx, const void* kernel, int grid, int threads, void** arg
 }
 
 int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, PcgVec<double> v, double scale,
-                  int max_iter, SolveCtl* out, int* launched) {
+                  int max_iter, int check_every, SolveCtl* out, int* launched) {
   *launched = 0;
   if (nslots <= 0 || ctx->num_sms < kPsGrid) return PF_OK;
   const int grid = std::min(nslots, kPsGrid), k = (nslots + kPsGrid - 1) / kPsGrid;
@@ -512,10 +513,11 @@ int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
   const bool resident = k <= kPsVirt;
   if (!resident && k * ps_slot_bytes() > room) return PF_OK;
   PsPlain a{nslots, std::min(nslots, kMaxRedBlocks), ctx->ctl, kind, nbr, v.x, v.r, v.p, v.z, v.diag, v.cx, v.cy,
-            v.cz, scale, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0};
+            v.cz, scale, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0, 0};
   while (!out->done && *launched < max_iter) {
+    a.turns = std::min(check_every > 0 ? check_every : kPsTurns, max_iter - *launched);
     a.tag = ctx->ps_tag + 1;
-    ctx->ps_tag += kPsChunk;
+    ctx->ps_tag += a.turns;
     bool refused = false;
     const int rc = resident ? launch_resident(ctx, a, k, grid, &refused) : launch_stream(ctx, a, k, grid, room, &refused);
     if (rc || refused) return rc;
@@ -523,7 +525,7 @@ int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
     PF_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     *out = *ctx->h_ctl;
     if (out->aux[0] != 0.0) return set_error(ctx, PF_ERR_CUDA, "pressure solve: a grid-wide wait ran out");
-    *launched += std::min(kPsChunk, max_iter - *launched);
+    *launched += a.turns;
   }
   return PF_OK;
 }

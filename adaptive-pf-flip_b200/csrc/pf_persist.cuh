@@ -44,7 +44,7 @@ constexpr int kPsVirt = kMaxRedBlocks / kPsGrid;    // virtual CTAs of one CTA, 
 constexpr unsigned kPsPolls = 1u << 22;
 constexpr int kPsWarps = PF_TV / 32;                // warps of a virtual CTA
 constexpr int kPsFace = 6 * 64;                     // face values of a slot
-constexpr int kPsChunk = 2048;                      // iterations per launch
+constexpr int kPsTurns = 2048;                      // iterations of a launch, if the caller names none
 
 static_assert(kMaxRedBlocks % kPsGrid == 0, "a CTA must own whole virtual CTAs");
 static_assert(kPsWarps == 16, "half a warp folds one virtual CTA");

@@ -29,6 +29,7 @@ struct PsMixed {
   PsBar bar;
   PsPair* faces;
   unsigned long long tag;
+  int turns;  // iterations of this launch, at most
 };
 
 __device__ __forceinline__ float ld16(const void* a, int is16, size_t i) {
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(PF_TV, 1) k_mixed_resident(PsMixed A) {
   const bool writes = (lane & (32 / N - 1)) == 0;
   bool alive = true;
   unsigned long long arrivals = 0;
-  for (int turn = 0; turn < kPsChunk && !sc.done; ++turn) {
+  for (int turn = 0; turn < A.turns && !sc.done; ++turn) {
     const int par = turn & 1;
     const unsigned long long tag = A.tag + turn;
     // ---- phase 1: p = z + beta p, A'p
@@ -240,15 +241,17 @@ int launch_mixed(pf_ctx* ctx, PsMixed& a, int k, int grid, bool* refused) {
 }  // namespace
 
 int mixed_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, float* e, float* r, const float* d,
-                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, SolveCtl* out, int* launched) {
+                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, int check_every,
+                  SolveCtl* out, int* launched) {
   const int k = (nslots + kPsGrid - 1) / kPsGrid, grid = std::min(nslots, kPsGrid);
   *launched = 0;
   if (nslots <= 0 || ctx->num_sms < kPsGrid || k > kPsVirt) return PF_OK;
   PsMixed a{nslots, std::min(nslots, kMaxRedBlocks), 1, cc16, cp16, ctx->ctl, kind, nbr, e, r, d, p,
-            {c[0], c[1], c[2]}, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0};
+            {c[0], c[1], c[2]}, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0, 0};
   while (!out->done && *launched < max_iter) {
+    a.turns = std::min(check_every > 0 ? check_every : kPsTurns, max_iter - *launched);
     a.tag = ctx->ps_tag + 1;
-    ctx->ps_tag += kPsChunk;
+    ctx->ps_tag += a.turns;
     bool refused = false;
     const int rc = launch_mixed(ctx, a, k, grid, &refused);
     if (rc || refused) return rc;
@@ -257,7 +260,7 @@ int mixed_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
     *out = *ctx->h_ctl;
     if (out->aux[0] != 0.0) return set_error(ctx, PF_ERR_CUDA, "pressure solve: a grid-wide wait ran out");
     a.first = 0;
-    *launched += std::min(kPsChunk, max_iter - *launched);
+    *launched += a.turns;
   }
   return PF_OK;
 }

@@ -410,17 +410,19 @@ int solve_inner_outer(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, co
 // solver drivers (pf_pcg.cu)
 int pcg_plain(pf_ctx* ctx, int nslots, int nred, const uint8_t* kind, PcgVec<double> vec, double scale,
               const pf_solve_cfg* cfg, SolveResult* res);
-// PLAIN as a persistent kernel (pf_persist.cu).  *launched: the iterations it was
+// PLAIN as a persistent kernel (pf_persist.cu), check_every iterations a launch (0:
+// its own choice).  *launched: the iterations it was
 // launched for, 0 when the system has too many slots for it or the device refuses
 // its first launch (nothing was done then).  When it returns PF_OK with neither
 // out->done nor max_iter reached, a later launch was refused: the vectors and the
 // control block are those after an update, and the next pass is the direction.
 int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, PcgVec<double> v, double scale,
-                  int max_iter, SolveCtl* out, int* launched);
+                  int max_iter, int check_every, SolveCtl* out, int* launched);
 // MIXED's inner solve (started by k_mixed_start) as a persistent kernel
 // (pf_persist_mixed.cu); *launched as above
 int mixed_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, float* e, float* r, const float* d,
-                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, SolveCtl* out, int* launched);
+                  void* p, bool cp16, const void* const c[3], bool cc16, int max_iter, int check_every,
+                  SolveCtl* out, int* launched);
 // One cooperative launch of a persistent kernel, its arrival counter cleared before.
 // *refused: the device has no place for all its CTAs at once (a part of the GPU is
 // set aside for another process, for one) or launches nothing cooperatively;

@@ -1,7 +1,7 @@
 """Runs a Python snippet in a process whose cooperative launches pass through a
 shim in front of the CUDA runtime (LD_PRELOAD): it can hold each launch back for
-a while, or let the first few through and answer the rest with the error a
-device without room for the grid gives.  The GPU sees ordinary launches only."""
+a while, or answer all of them, or every second one, with the error a device
+without room for the grid gives.  The GPU sees ordinary launches only."""
 import os
 import subprocess
 import sys
@@ -15,16 +15,14 @@ SOURCE = r"""
 #include <unistd.h>
 typedef struct { unsigned x, y, z; } dim3_;
 typedef int (*launch_fn)(const void*, dim3_, dim3_, void**, size_t, void*);
-static int allowed = -2, delay_us;
+static int refuse_every = -1, delay_us, count;
 int cudaLaunchCooperativeKernel(const void* f, dim3_ g, dim3_ b, void** a, size_t smem, void* stream) {
-  if (allowed == -2) {
-    const char *n = getenv("COOP_ALLOW"), *d = getenv("COOP_DELAY_US");
-    delay_us = d ? atoi(d) : 0;
-    allowed = n ? atoi(n) : -1;
+  if (refuse_every < 0) {
+    delay_us = atoi(getenv("COOP_DELAY_US"));
+    refuse_every = atoi(getenv("COOP_REFUSE_EVERY"));
   }
   if (delay_us) usleep(delay_us);
-  if (allowed == 0) return 720; /* cudaErrorCooperativeLaunchTooLarge */
-  if (allowed > 0) --allowed;
+  if (refuse_every && ++count % refuse_every == 0) return 720; /* cudaErrorCooperativeLaunchTooLarge */
   void* rt = dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD);
   if (!rt) return 999;
   launch_fn real = (launch_fn)dlsym(rt, "cudaLaunchCooperativeKernel");
@@ -33,14 +31,11 @@ int cudaLaunchCooperativeKernel(const void* f, dim3_ g, dim3_ b, void** a, size_
 """
 
 
-def run_under_shim(tmp_path, code, allow=None, delay_us=0, timeout=300):
+def run_under_shim(tmp_path, code, refuse_every=0, delay_us=0, timeout=300):
     src, so = tmp_path / "coop_shim.c", tmp_path / "coop_shim.so"
     src.write_text(SOURCE)
     subprocess.run(["gcc", "-shared", "-fPIC", "-O1", str(src), "-o", str(so), "-ldl"], check=True)
-    env = dict(os.environ, LD_PRELOAD=str(so), COOP_DELAY_US=str(delay_us))
-    env.pop("COOP_ALLOW", None)
-    if allow is not None:
-        env["COOP_ALLOW"] = str(allow)
+    env = dict(os.environ, LD_PRELOAD=str(so), COOP_DELAY_US=str(delay_us), COOP_REFUSE_EVERY=str(refuse_every))
     env["PYTHONPATH"] = os.pathsep.join([os.path.join(ROOT, "tests"), ROOT] +
                                         [p for p in [env.get("PYTHONPATH")] if p])
     out = subprocess.run([sys.executable, "-c", code], env=env, cwd=ROOT, capture_output=True, text=True,

@@ -232,7 +232,7 @@ def test_mr_refused_launch_leaves_the_work_to_the_kernels_per_iteration(pf, tmp_
     atomics leave 1e-6 of the scale)."""
     from coop_shim import run_under_shim
     path = str(tmp_path / "mr.npz")
-    run_under_shim(tmp_path, MR_STEP.format(path=path, iters=12), allow=0)
+    run_under_shim(tmp_path, MR_STEP.format(path=path, iters=12), refuse_every=1)
     refused = np.load(path)
     p, st = chained_step(pf, 12)
     assert np.array_equal(st[:3], refused["st"][:3]) and st[2] == 12

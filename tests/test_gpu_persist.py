@@ -220,5 +220,43 @@ def test_refused_launches_leave_the_work_to_the_kernels_per_iteration(pf, tmp_pa
     bits, PLAIN at every way its slots are kept and MIXED in its three storages."""
     from coop_shim import run_under_shim
     path = str(tmp_path / "refused.npz")
-    run_under_shim(tmp_path, SOLVE_ALL.format(path=path, check_every=0), allow=0)
+    run_under_shim(tmp_path, SOLVE_ALL.format(path=path, check_every=0), refuse_every=1)
+    _same_bits(solve_all(pf), dict(np.load(path)))
+
+
+@pytest.mark.parametrize("mode", ["plain", "mixed"])
+@pytest.mark.parametrize("shape", [(39, 30, 22), (88, 86, 81)], ids=str)
+def test_check_every_is_the_iterations_of_a_launch(pf, shape, mode):
+    """The host looks at the solve every check_every iterations: one launch for each."""
+    g = pf.SparseMacGrid3D(*shape, 1.0 / max(shape), max_particles=int(np.prod(shape)) // 4 + 64)
+    fields = _system(shape, sum(shape), solids=False)
+    counts = []
+    for check_every in (0, 6, 1):
+        for f, v in fields.items():
+            g.set_field(f, v, np.ones(g.bdims(f)[::-1], np.uint8))
+        cfg = pf.SolverConfig(check_every=check_every) if mode == "plain" else pf.SolverConfig(
+            mode=pf.PF_SOLVER_MIXED, check_every=check_every, inner_rel_tol=1e-30, inner_max_iter=12)
+        before = g.lib.pf_launch_count(g.ctx)
+        st = pf.spProjectStepVC3D(g, pf.PhaseParams(1.0, 0.01), 1.0 / 60, 12, 0.0, 0.01, solver=cfg)
+        assert st.iterations == 12
+        counts.append(g.lib.pf_launch_count(g.ctx) - before)
+    g.close()
+    if mode == "mixed" and max(shape) > 80:  # three launches per iteration, however often the host looks
+        assert counts[1] == counts[0] and counts[2] == counts[0]
+    else:
+        assert [c - counts[0] for c in counts] == [0, 1, 11]
+
+
+def test_launches_chain_with_the_same_bits(pf):
+    """Seven iterations a launch against all in one, for every kernel that runs a
+    solve in launches: the vectors, scalars, faces and tags pass from one to the next."""
+    _same_bits(solve_all(pf), solve_all(pf, check_every=7))
+
+
+def test_a_launch_refused_in_mid_solve(pf, tmp_path):
+    """A solve's first launch runs seven iterations, its second is refused, and the
+    kernels per iteration take over: the same bits."""
+    from coop_shim import run_under_shim
+    path = str(tmp_path / "taken_over.npz")
+    run_under_shim(tmp_path, SOLVE_ALL.format(path=path, check_every=7), refuse_every=2)
     _same_bits(solve_all(pf), dict(np.load(path)))
