@@ -515,7 +515,7 @@ int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
   PsPlain a{nslots, std::min(nslots, kMaxRedBlocks), ctx->ctl, kind, nbr, v.x, v.r, v.p, v.z, v.diag, v.cx, v.cy,
             v.cz, scale, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0, 0};
   while (!out->done && *launched < max_iter) {
-    a.turns = std::min(check_every > 0 ? check_every : kPsTurns, max_iter - *launched);
+    a.turns = std::min(check_every > 0 ? check_every : resident ? kPsTurns : kPsStreamTurns / k, max_iter - *launched);
     a.tag = ctx->ps_tag + 1;
     ctx->ps_tag += a.turns;
     bool refused = false;

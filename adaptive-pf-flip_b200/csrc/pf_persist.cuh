@@ -32,6 +32,13 @@
 // Each reduction has two sets of entries, used alternately: a CTA that writes
 // a set again has passed the reduction in between, so every CTA has read it.
 //
+// One launch holds every SM: a kernel of another stream (an asynchronous upload's
+// unpacking, another context's work, the caller's own) starts only when it ends.
+// So a launch runs no more than kPsTurns iterations of the resident kernels, and
+// kPsStreamTurns / k where they take about 1.8 k us for the k slots of a CTA: 8 ms
+// or less (2000 iterations in one launch held 11 ms at 48^3, 99 at 128^3, 173 at
+// 148^3).  A launch more costs 15 us up to 64^3 and 50 at 128^3, under 1 % of that.
+//
 // Every wait is bounded (kPsPolls polls); a CTA that runs out of them sets
 // SolveCtl::aux[0] and leaves, and the host returns an error.
 #pragma once
@@ -41,10 +48,10 @@
 namespace pf {
 
 constexpr int kPsVirt = kMaxRedBlocks / kPsGrid;    // virtual CTAs of one CTA, at most
+constexpr int kPsTurns = 1024, kPsStreamTurns = 4 * kPsTurns;
 constexpr unsigned kPsPolls = 1u << 22;
 constexpr int kPsWarps = PF_TV / 32;                // warps of a virtual CTA
 constexpr int kPsFace = 6 * 64;                     // face values of a slot
-constexpr int kPsTurns = 2048;                      // iterations of a launch, if the caller names none
 
 static_assert(kMaxRedBlocks % kPsGrid == 0, "a CTA must own whole virtual CTAs");
 static_assert(kPsWarps == 16, "half a warp folds one virtual CTA");

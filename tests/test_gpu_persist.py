@@ -260,3 +260,42 @@ def test_a_launch_refused_in_mid_solve(pf, tmp_path):
     path = str(tmp_path / "taken_over.npz")
     run_under_shim(tmp_path, SOLVE_ALL.format(path=path, check_every=7), refuse_every=2)
     _same_bits(solve_all(pf), dict(np.load(path)))
+
+
+def test_other_streams_run_between_the_launches(pf):
+    """While a long solve runs, a small kernel on another stream waits for a launch
+    of the solve at most, not for the solve: the longest wait is under half of the
+    solve's device time."""
+    import threading
+    import time
+
+    import torch
+    n, its = 96, 3000
+    sc = pf.scenes.ellipsoid_pressure(n, seed=1)
+    pp = pf.PhaseParams(sc["rho_l"], sc["rho_g"])
+    g = pf.SparseMacGrid3D(n, n, n, sc["dx"], max_particles=n ** 3 // 4)
+    pp.rho_tilde_0 = pf.calibrateRhoTilde0(pp, 1.0, grid=g)
+    names = ("u", "v", "w", "mu", "mv", "mw", "p", "mk")
+    fields = pf.scenes.pressure_grid_fields(sc, pp.rho_tilde_0)
+    for k, v in fields.items():
+        if k in names:
+            f = names.index(k)
+            g.set_field(f, v, np.ones(g.bdims(f)[::-1], np.uint8))
+    side, x = torch.cuda.Stream(), torch.zeros(1, device="cuda")
+    with torch.cuda.stream(side):
+        x += 1
+    side.synchronize()
+    st = []
+    t = threading.Thread(target=lambda: st.append(pf.spProjectStepVC3D(g, pp, 1.0 / 240, its, 0.0)))
+    t.start()
+    longest = 0.0
+    while t.is_alive():
+        t0 = time.perf_counter()
+        with torch.cuda.stream(side):
+            x += 1
+        side.synchronize()
+        longest = max(longest, 1e3 * (time.perf_counter() - t0))
+    t.join()
+    assert st[0].iterations == its
+    assert longest < 0.5 * st[0].solve_ms, (longest, st[0].solve_ms)
+    g.close()
