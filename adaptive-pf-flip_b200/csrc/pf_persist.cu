@@ -13,6 +13,7 @@
 
 #include "pf_ctx.h"
 #include "pf_persist.cuh"
+#include "pf_quotient.cuh"
 
 namespace pf {
 namespace {
@@ -30,25 +31,6 @@ struct PsPlain {
   unsigned long long tag;
   int turns;      // iterations of this launch, at most
 };
-
-// r / d, correctly rounded, from inv = RN(1 / d) formed once per solve: the
-// product and two residual corrections (Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990:
-// with a correctly rounded reciprocal the correction of a faithful quotient is
-// correctly rounded; the first correction makes the product faithful).  Every
-// step is exact enough only while nothing nears the ends of the exponent range,
-// so a cell whose d is outside 2^+-400 has inv = 0, and that or an r outside
-// 2^+-500 takes the division (r = 0 gives 0 either way).  Five dependent
-// operations without a branch, where the division's take the throughput of
-// about 13.
-__device__ __forceinline__ double inv_of(double d) { return d > 0x1p-400 && d < 0x1p400 ? __ddiv_rn(1.0, d) : 0.0; }
-__device__ __forceinline__ double quotient(double r, double d, double inv) {
-  const double ar = fabs(r);
-  if (!(inv != 0.0 && ((ar > 0x1p-500 && ar < 0x1p500) || ar == 0.0))) return d > 0.0 ? __ddiv_rn(r, d) : 0.0;
-  double q = __dmul_rn(r, inv);
-  q = __fma_rn(__fma_rn(-q, d, r), inv, q);
-  return __fma_rn(__fma_rn(-q, d, r), inv, q);
-}
 
 // ---- everything on chip ---------------------------------------------------
 
