@@ -10,8 +10,8 @@ import oracle as O
 needs_ref = pytest.mark.skipif(not O.reference_available(), reason="oracle/_ref not built")
 
 
-def stepped_pair(n, seed, air=0.0, rho=(1000.0, 1.0)):
-    """Oracle and reference grids holding the same markers and P2G fields."""
+def stepped_oracle(n, seed, air=0.0, rho=(1000.0, 1.0)):
+    """An oracle grid holding the markers and P2G fields of a seeded scene."""
     rng = np.random.default_rng(seed)
     dx = 1.0 / n
     pos = rng.uniform(0.6 * dx, 1 - 0.6 * dx, (30 * n ** 2, 3)).astype(np.float32).astype(np.float64)
@@ -22,10 +22,17 @@ def stepped_pair(n, seed, air=0.0, rho=(1000.0, 1.0)):
     ps = O.Particles(pos, vel, typ, rng.uniform(0.5, 1.5, len(pos)))
     pp = O.PhaseParams(*rho)
     pp.rho_tilde_0 = O.Oracle().calibrate_rho_tilde0(pp, 1.0)
-    go, gr = O.OracleGrid(n, n, n, dx), O.ReferenceGrid(n, n, n, dx)
+    go = O.OracleGrid(n, n, n, dx)
     o = O.Oracle()
     o.mark_cells(go, ps)
     o.p2g(go, ps, pp, 1.0)
+    return go, pp
+
+
+def stepped_pair(n, seed, air=0.0, rho=(1000.0, 1.0)):
+    """Oracle and reference grids holding the same markers and P2G fields."""
+    go, pp = stepped_oracle(n, seed, air, rho)
+    gr = O.ReferenceGrid(n, n, n, 1.0 / n)
     for f in range(8):
         gr.set_field(f, *go.get_field(f))
     return go, gr, pp

@@ -11,7 +11,7 @@ import pytest
 
 import oracle as O
 from gpu_helpers import scene_particles
-from test_diag_oracle import stepped_pair
+from test_diag_oracle import stepped_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -30,7 +30,7 @@ def _check(gs, os_):
 
 @pytest.mark.parametrize("n,seed,air", [(8, 1, 0.0), (12, 2, 0.3), (16, 3, 0.5), (24, 7, 0.2)])
 def test_interface_diagnostics_match_oracle(pf, n, seed, air):
-    go, _, pp = stepped_pair(n, seed, air)
+    go, pp = stepped_oracle(n, seed, air)
     g = pf.SparseMacGrid3D(n, n, n, 1.0 / n)
     for f in range(8):
         g.set_field(f, *go.get_field(f))
@@ -74,7 +74,7 @@ def test_step_records_diagnostics_after_p2g(pf):
 def test_surface_tension_matches_oracle(pf, n, seed, air, strength, maxdv, radius):
     """applySparseSurfaceTension3D: face velocities equal the oracle's bit for
     bit; counts, flags and maxima exact, means within 1e-12."""
-    go, _, pp = stepped_pair(n, seed, air)
+    go, pp = stepped_oracle(n, seed, air)
     g = pf.SparseMacGrid3D(n, n, n, 1.0 / n)
     for f in range(8):
         g.set_field(f, *go.get_field(f))

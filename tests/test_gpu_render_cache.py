@@ -90,7 +90,6 @@ def _expected_particles(ps, Vp):
     return out
 
 
-@pytest.mark.skipif(not O.reference_available(), reason="compiled reference (oracle/_ref) not built")
 def _secondary_sets(rng, n):
     out = []
     for m in (140, 60):
@@ -103,6 +102,7 @@ def _secondary_sets(rng, n):
     return out
 
 
+@pytest.mark.skipif(not O.reference_available(), reason="compiled reference (oracle/_ref) not built")
 @pytest.mark.parametrize("scene,n,seed,secondary", [("rayleigh_taylor", 16, 3, False), ("bubble_tank", 20, 5, False),
                                                     ("bubble_tank", 20, 7, True)])
 def test_render_cache_equals_reference_writer(pf, tmp_path, scene, n, seed, secondary):
