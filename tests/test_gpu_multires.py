@@ -203,27 +203,30 @@ MR_STEP = """
 import sys
 import numpy as np
 from conftest import load_package
-from test_gpu_multires import chained_step
-pf = load_package()
-p, st = chained_step(pf, {iters})
-np.savez({path!r}, p=p, st=st)
+from test_gpu_multires import one_step
+np.savez({path!r}, *one_step(load_package(), *{args}))
 """
 
 
-def chained_step(pf, iters):
-    """One step of a two-level tank whose pressure system takes `iters` iterations."""
-    n = 40
-    s = MRSettings(dt=1 / 60, phase=_phase(), dynamic_refinement=False, cg_iters=iters, cg_rel_tol=0.0, cg_tol=0.0)
+def one_step(pf, n, ratio, iters, rel_tol, fine):
+    """One step of a tank of water full of gas bubbles, refined up to z = `fine`; the
+    pressure and what its solve reports."""
+    phase = O.PhaseParams(1.0, 1.0 / ratio)
+    phase.rho_tilde_0 = O.Oracle().calibrate_rho_tilde0(phase, 1.0)
+    s = MRSettings(dt=1 / 60, phase=phase, dynamic_refinement=False, cg_iters=iters, cg_rel_tol=rel_tol, cg_tol=0.0)
     rng = np.random.default_rng(3)
     k, j, i = np.meshgrid(np.arange(1, n - 1), np.arange(1, n - 6), np.arange(1, n - 1), indexing="ij")
     cells = np.stack([i.ravel(), j.ravel(), k.ravel()], 1)
     pos = ((cells + rng.uniform(0.1, 0.9, cells.shape)) / n).astype(np.float32)
     vel = rng.normal(0, 0.3, pos.shape).astype(np.float32)
-    sim, _ = _pair(pf, (n, n, n), 1.0 / n, s, pos, vel, np.zeros(len(pos), np.uint8), boxes=[(0, 0, 0, n, n, 16)])
+    gas = np.zeros(len(pos), np.uint8)
+    for c in rng.uniform(0, 1, (24, 3)):
+        gas |= (((pos - c) ** 2).sum(1) < 0.08 ** 2).astype(np.uint8)
+    sim, _ = _pair(pf, (n, n, n), 1.0 / n, s, pos, vel, gas, boxes=[(0, 0, 0, n, n, fine)])
     st = sim.step()
     p = sim.cells()[1]
     sim.close()
-    return p, np.array([st.active_cells, st.pinned_cell, st.iterations, st.final_residual])
+    return p, np.array([st.active_cells, st.pinned_cell, st.iterations, st.converged])
 
 
 def test_mr_refused_launch_leaves_the_work_to_the_kernels_per_iteration(pf, tmp_path):
@@ -231,9 +234,28 @@ def test_mr_refused_launch_leaves_the_work_to_the_kernels_per_iteration(pf, tmp_
     orders: pressures after a few iterations agree as those of two runs do (P2G's
     atomics leave 1e-6 of the scale)."""
     from coop_shim import run_under_shim
-    path = str(tmp_path / "mr.npz")
-    run_under_shim(tmp_path, MR_STEP.format(path=path, iters=12), refuse_every=1)
-    refused = np.load(path)
-    p, st = chained_step(pf, 12)
-    assert np.array_equal(st[:3], refused["st"][:3]) and st[2] == 12
-    assert rel_err(p, refused["p"]) < 1e-5
+    path, args = str(tmp_path / "mr.npz"), (40, 1.0, 12, 0.0, 16)
+    run_under_shim(tmp_path, MR_STEP.format(path=path, args=args), refuse_every=1)
+    q, refused = np.load(path).values()
+    p, st = one_step(pf, *args)
+    assert np.array_equal(st, refused) and st[2] == 12
+    assert rel_err(p, q) < 1e-5
+
+
+def test_mr_solves_of_more_than_one_launch(pf, tmp_path):
+    """A solve of more than the 512 iterations of a launch: in launches, in one
+    launch and then by the kernels per iteration, and by those alone.  All converge,
+    and in as many iterations: one that lost its direction between two launches
+    would start over there.  The pressures agree within the residual (1e-9) times a
+    condition number of some 2e6 (a contrast of 1000 on 48 cells an axis)."""
+    from coop_shim import run_under_shim
+    args = (48, 1000.0, 6000, 1e-9, 48)
+    p, st = one_step(pf, *args)
+    assert st[3] == 1 and st[2] > 512
+    for refuse_every in (1, 2):
+        path = str(tmp_path / f"mr{refuse_every}.npz")
+        run_under_shim(tmp_path, MR_STEP.format(path=path, args=args), refuse_every=refuse_every)
+        q, other = np.load(path).values()
+        assert np.array_equal(st[[0, 1, 3]], other[[0, 1, 3]])
+        assert abs(st[2] - other[2]) <= 0.1 * other[2], (st, other)
+        assert rel_err(p, q) < 2e-3
