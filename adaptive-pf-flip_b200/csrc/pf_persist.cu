@@ -2,13 +2,16 @@
 // pf_persist.cuh for the reductions and the grid-wide barriers).
 //
 // Two kernels, by the slots a CTA owns (k = ceil(nslots / 148)): k_plain_resident
-// for k <= 8 (up to 1184 slots, e.g. 80^3 cells), k_plain_stream while a slot's
-// 4.6 KB of shared memory fit (k <= 49, e.g. 150^3); larger systems take the
-// three kernels of pf_pcg.cu.  Every operation rounds as there and the sums run
+// for k <= 6 (up to 888 slots, e.g. 71^3 cells), k_plain_stream while a slot's
+// 4.6 KB of shared memory fit (k <= 49, e.g. 150^3); larger systems, and a device
+// that refuses the cooperative launch, take the three kernels of pf_pcg.cu.  Every operation rounds as there and the sums run
 // in the same order, so x, the iteration count and the residuals have the same
 // bits.  Per iteration, before (three launches) and now: 24^3 cells 21 -> 4.4 us,
 // 48^3 25 -> 5.6, 64^3 28.6 -> 7.7, 128^3 80 -> 51.  Where the streaming kernel
 // ends, 148^3 takes 87 us and the three kernels at 152^3 101: 93 for as many cells.
+// Where the resident one ends (tiles: us resident, streaming): 544: 6.4, 10.4; 704:
+// 7.7, 11.1; 810: 8.7, 12.7; with a kernel of eight slots, which spills, 900: 14.1,
+// 13.2; 972: 13.1, 12.9; 1000: 14.6, 13.5.
 #include <algorithm>
 
 #include "pf_ctx.h"
@@ -45,6 +48,7 @@ struct PsPlain {
 // its six neighbour faces), the couplings (13.5 KB with the high faces') and x
 // (4 KB).  512 threads: more would leave under 128 registers, and the U independent
 // slots of a thread hide its latencies as well as more warps would.
+constexpr int kResSlots = 6;
 constexpr int kResSlotDoubles = 2 * PF_TV + kPsFace + 3 * PF_TV + 3 * 64;
 
 template <int U>
@@ -453,8 +457,7 @@ int launch_resident(pf_ctx* ctx, PsPlain& a, int k, int grid, bool* refused) {
     case 2: return launch_resident<2>(ctx, a, grid, refused);
     case 3: return launch_resident<3>(ctx, a, grid, refused);
     case 4: return launch_resident<4>(ctx, a, grid, refused);
-    case 5: case 6: return launch_resident<6>(ctx, a, grid, refused);
-    default: return launch_resident<8>(ctx, a, grid, refused);
+    default: return launch_resident<kResSlots>(ctx, a, grid, refused);
   }
 }
 
@@ -492,7 +495,7 @@ int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
   if (nslots <= 0 || ctx->num_sms < kPsGrid) return PF_OK;
   const int grid = std::min(nslots, kPsGrid), k = (nslots + kPsGrid - 1) / kPsGrid;
   const size_t room = ctx->smem_optin - sizeof(PsShared) - 64;
-  const bool resident = k <= kPsVirt;
+  const bool resident = k <= kResSlots;
   if (!resident && k * ps_slot_bytes() > room) return PF_OK;
   PsPlain a{nslots, std::min(nslots, kMaxRedBlocks), ctx->ctl, kind, nbr, v.x, v.r, v.p, v.z, v.diag, v.cx, v.cy,
             v.cz, scale, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0, 0};

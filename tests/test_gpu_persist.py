@@ -1,8 +1,8 @@
 """The PLAIN solve at every way its work is split over the GPU, and the other modes beside it.
 
-A system's tiles go to 148 CTAs: one to eight tiles each live on chip (a kernel
-per count, 5 and 7 running in the next larger one's), more are streamed with as
-many of r and x on chip as fit, and beyond about 7200 tiles three kernels run
+A system's tiles go to 148 CTAs: one to six tiles each live on chip (a kernel per
+count, 5 running in the next larger one's; MIXED up to eight), more are streamed
+with as many of r and x on chip as fit, and beyond about 7200 tiles three kernels run
 per iteration.  The grids below take one of each, ragged ones among them, with
 solid, empty and fluid cells mixed.
 
@@ -173,9 +173,10 @@ def test_two_threads_solve_side_by_side(pf, tmp_path):
     run_under_shim(tmp_path, THREADS, delay_us=3000)
 
 
-# one slot a CTA, five and seven in the next larger kernels, eight, streaming with
-# r and x kept and with part of them kept
-BITS = [((39, 30, 22), (0, 1, 2)), ((70, 71, 72), (0, 2)), ((78, 79, 72), ()), ((80, 79, 77), (0, 1, 2)),
+# one to six slots a CTA (on chip), seven and eight (PLAIN streams them, MIXED's live on
+# chip), streaming with r and x kept and with part of them kept
+BITS = [((39, 30, 22), (0, 1, 2)), ((46, 47, 40), ()), ((54, 55, 62), ()), ((63, 62, 56), ()), ((64, 64, 64), ()),
+        ((70, 71, 72), (0, 2)), ((78, 79, 72), (1,)), ((80, 79, 77), (0, 1, 2)),
         ((88, 86, 81), ()), ((127, 118, 100), ())]
 
 
