@@ -72,9 +72,9 @@ SPLAT_WARP_INST_PER_PARTICLE = 42.1
 # kind / coarse-class bytes 1 B); a neighbour's value is an L1/L2 hit and is
 # not counted again.
 PCG_BYTES = {
-    # the three-kernel path (256^3): k_spmv_plain_tab 49 (p, 3 couplings, diagonal, kind, Ap), k_update_plain 65,
-    # k_direction_plain 25; up to about 150^3 one persistent kernel keeps part of the vectors on chip
-    "plain": 139,
+    "plain": 139,            # three kernels: k_spmv_plain_tab 49 (p, 3 couplings, diagonal, kind, Ap),
+                             # k_update_plain 65, k_direction_plain 25
+    "plain_stream": 96,      # k_plain_stream with neither r nor x on chip: p 24, x 16, couplings 24, diagonal 16, r 16
     "flex64": 133,           # k_fx_spmv 49, k_fx_update 34, k_fx_dir 50 (the learned coarse path is not HBM-bound)
     "inner_fp32": 71,        # k_mixed_spmv 25, k_mixed_update 29, k_mixed_direction 17
     "inner_bf16": 65,        # the same with BF16 couplings
@@ -82,26 +82,51 @@ PCG_BYTES = {
     "inner_learned32": 69,   # FP32 k_fx_spmv 25, k_fx_update 18, k_fx_dir 26
     "outer": 165,            # per outer FCG(1) iteration: k_oc_beta 13, k_oc_dir 21, k_oc_spmv 57, k_oc_update 49, inner start 25
 }
+# Which kernels run, by the tiles each of the 148 CTAs of a persistent solve has
+# (csrc/pf_persist.cu, csrc/pf_persist_mixed.cu).  The streaming kernel has 230,912 B
+# of shared memory for 4,640 B a tile and, as far as they fit, r and x at 4 KB each.
+PLAIN_ON_CHIP_TILES, MIXED_ON_CHIP_TILES = 6, 8
+STREAM_ROOM, STREAM_SLOT, STREAM_VECTOR = 230912, 4640, 4096
 
 
-def pcg_bytes(pf, cfg, st):
-    """Algorithmic bytes per unknown of one solve (PCG_BYTES x iterations)."""
+def plain_bytes(tiles):
+    """Bytes per unknown and iteration of a PLAIN solve over `tiles` pooled
+    tiles; None where its vectors stay on chip."""
+    k = -(-tiles // 148)
+    if k <= PLAIN_ON_CHIP_TILES:
+        return None
+    if k * STREAM_SLOT > STREAM_ROOM:
+        return PCG_BYTES["plain"]
+    kept = min(2 * k, (STREAM_ROOM - k * STREAM_SLOT) // STREAM_VECTOR)
+    return PCG_BYTES["plain_stream"] - 16.0 * kept / k  # r or x of a kept tile is neither read nor written
+
+
+def pcg_bytes(pf, cfg, st, tiles):
+    """Algorithmic bytes per unknown of one solve (bytes per iteration x
+    iterations); None for a solve that keeps its vectors on chip."""
     if cfg.mode == pf.PF_SOLVER_PLAIN:
-        return PCG_BYTES["plain"] * st.iterations
+        b = plain_bytes(tiles)
+        return None if b is None else b * st.iterations
     if cfg.mode == pf.PF_SOLVER_LEARNED and not cfg.inner_fp32:
         return PCG_BYTES["flex64"] * st.iterations
     if cfg.mode == pf.PF_SOLVER_LEARNED:
         inner = PCG_BYTES["inner_learned32"]
+    elif -(-tiles // 148) <= MIXED_ON_CHIP_TILES:
+        return None
     else:
         inner = PCG_BYTES[{0: "inner_fp32", 1: "inner_bf16"}.get(int(cfg.bf16_storage), "inner_bf16_dir")]
     return inner * st.iterations + PCG_BYTES["outer"] * st.refinements
 
 
-def pcg_roofline(pf, cfg, st, peak):
-    """Achieved bytes/s of a solve's fine-level passes against the HBM peak."""
-    b = pcg_bytes(pf, cfg, st) * st.n_cells
-    gbs = b / max(st.solve_ms / 1000.0, 1e-12) / 1e9
-    return {"bytes_per_unknown": pcg_bytes(pf, cfg, st), "achieved_gbs": gbs, "frac": gbs / peak}
+def pcg_roofline(pf, cfg, st, tiles, peak):
+    """Achieved bytes/s of a solve's fine-level passes against the HBM peak; for
+    a solve on chip, bound by its grid-wide sums, its time per iteration only."""
+    per = pcg_bytes(pf, cfg, st, tiles)
+    if per is None:
+        return {"bound": "grid-wide sums (vectors on chip)",
+                "us_per_iteration": 1e3 * st.solve_ms / max(st.iterations, 1)}
+    gbs = per * st.n_cells / max(st.solve_ms / 1000.0, 1e-12) / 1e9
+    return {"bytes_per_unknown": per, "achieved_gbs": gbs, "frac": gbs / peak}
 
 
 def issue_roofline(n_particles, splat_ms, sm_mhz, sms=148, schedulers=4):
@@ -448,7 +473,8 @@ def run_pcg(pf, n, modes, max_iter=20000, seed=0, weights_path=None, fp64_oracle
         p, _ = g.get_field(pf.PF_P)
         rec = {"ms_to_1e-6": st.solve_ms, "iterations": st.iterations, "refinements": st.refinements,
                "converged": bool(st.converged), "rel_residual": st.res_final / max(st.res0, 1e-300),
-               "setup_ms": tm.as_dict()["precond_setup"][0], "roofline": pcg_roofline(pf, cfg, st, peak)}
+               "setup_ms": tm.as_dict()["precond_setup"][0],
+               "roofline": pcg_roofline(pf, cfg, st, lib.pf_active_tiles(g.ctx), peak)}
         if cfg.mode == pf.PF_SOLVER_LEARNED:
             rec["coarse_accepted"] = st.precond_applied
             rec["coarse_rejected"] = st.precond_rejected
@@ -528,7 +554,8 @@ def run_step_pcg(pf, name, n, modes, pre_steps=1, max_iter=20000, seed=0, weight
         stages = tm.as_dict()
         rec = {"ms_to_1e-6": st.solve_ms, "iterations": st.iterations, "refinements": st.refinements,
                "converged": bool(st.converged), "rel_residual": st.res_final / max(st.res0, 1e-300),
-               "setup_ms": stages["precond_setup"][0], "roofline": pcg_roofline(pf, cfg, st, peak)}
+               "setup_ms": stages["precond_setup"][0],
+               "roofline": pcg_roofline(pf, cfg, st, lib.pf_active_tiles(sim.grid.ctx), peak)}
         if cfg.mode == pf.PF_SOLVER_LEARNED:
             tot = st.precond_applied + st.precond_rejected
             rec["coarse_accepted"] = st.precond_applied
