@@ -841,9 +841,12 @@ __global__ void __launch_bounds__(kMrNT) k_mr_update(int N, MrVecs V, MrCtl* ctl
 //   update     x, r, z, r.z, max|r|         reduction B (and one for r.(z - z_prev)
 //                                           with the flexible beta)
 // The columns and coefficients are kept in shared memory, whole slices as far as
-// they fit, so a row waits for one round of gathers instead of two.  As two
-// launches per iteration with last-CTA reductions, an iteration of the 128^3 dam
-// break (142k rows) took 19 us; here 9.1, two thirds of it the three barriers.
+// they fit, so a row waits for one round of gathers instead of two.  Per iteration,
+// as two launches with last-CTA reductions and here (dam breaks; rows: us): one row
+// a thread 4.8k: 15.5, 8.6; 48k: 16.9, 8.8; 142k: 18.8, 9.4; two 276k: 22.1, 13.1;
+// three 409k: 24.8, 17.2.  Two thirds of it at one row are the three barriers (the
+// barrier stall is 17 of 29 cycles per issue); two and three rows spill 152 and 324
+// bytes at 64 registers and still win.  Four would not fit the registers.
 // The scalar rules are mr_finalize's, applied by every thread to its own copy;
 // the inner products add up in another fixed order.
 constexpr int kMrResNT = 1024, kMrResRows = 3;
@@ -1537,7 +1540,7 @@ int project_mr(pf_ctx* ctx, MrState* s, const pf_mr_step_cfg* cfg, pf_mr_step_st
     PsBar bar{ctx->ps_entries, ctx->ps_counter};
     while (!c.done && launched < cfg->cg_iters) {
       unsigned long long tag = ctx->ps_tag + 1;
-      int turns = std::min(kPsTurns / 2, cfg->cg_iters - launched);  // 9 to 17 us each
+      int turns = std::min(kPsTurns / 4, cfg->cg_iters - launched);  // 9 to 17 us each
       ctx->ps_tag += 2 * turns;
       int n = N, first = launched == 0;
       const int *sp = s->slice_ptr, *cl = s->col, *ar = tot + 3;

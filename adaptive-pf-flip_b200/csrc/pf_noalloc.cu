@@ -14,9 +14,10 @@
 // It runs pf_project's PLAIN set-up, Jacobi-PCG recurrences and velocity
 // update (the launchers in pf_project.cu and pf_pcg.cu) on a pool in which
 // every tile is active.  Its SpMV finds cross-tile neighbours through the tile
-// map in shared memory (k_spmv_plain); pf_project's PLAIN solve reads them
-// from a per-solve neighbour-slot table (k_spmv_plain_tab), which would need
-// memory this entry point does not have.  Both give the same rows.
+// map in shared memory (k_spmv_plain); pf_project's PLAIN solves (pf_persist.cu
+// for grids of this size, k_spmv_plain_tab above) read them from a per-solve
+// neighbour-slot table, which would need memory this entry point does not have.
+// All give the same rows, and the same sums in the same order.
 #include <cmath>
 #include <cstring>
 

@@ -2,10 +2,11 @@
 //
 // PLAIN: FP64 Jacobi-PCG with the reference's recurrences and stopping rule
 //   (src/driver/sparse_ops3d_tp.cpp:315-364).  Systems of up to about 7200 tiles
-//   run in a persistent kernel (pf_persist.cu); larger ones, and the
-//   allocation-free projection, take three kernels per iteration: SpMV + p.Ap,
-//   x/r update + r.z + max|r|, direction update.  There the 139 bytes a cell and
-//   iteration bound the time (0.51 ms at 256^3, 0.70 of the copy bandwidth).
+//   run in a persistent kernel (pf_persist.cu); larger ones, those of a device that
+//   refuses its launch, and the allocation-free projection take three kernels per
+//   iteration: SpMV + p.Ap, x/r update + r.z + max|r|, direction update.  There the
+//   139 bytes a cell and iteration bound the time (0.42 ms at 256^3, 0.84 of the
+//   copy bandwidth).
 // MIXED: FP64 outer iterative refinement r = b - A x with the exact FP64
 //   operator, inner Jacobi-PCG with FP32 vectors and FP32 (or BF16) scaled
 //   face coefficients, FP64 inner products and norms.  The BF16 operator keeps

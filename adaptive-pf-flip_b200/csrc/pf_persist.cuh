@@ -35,9 +35,10 @@
 // One launch holds every SM: a kernel of another stream (an asynchronous upload's
 // unpacking, another context's work, the caller's own) starts only when it ends.
 // So a launch runs no more than kPsTurns iterations of the resident kernels, and
-// kPsStreamTurns / k where they take about 1.8 k us for the k slots of a CTA: 8 ms
+// kPsStreamTurns / k where they take about 1.8 k us for the k slots of a CTA: 16 ms
 // or less (2000 iterations in one launch held 11 ms at 48^3, 99 at 128^3, 173 at
-// 148^3).  A launch more costs 15 us up to 64^3 and 50 at 128^3, under 1 % of that.
+// 148^3).  A launch more costs 15 us up to 64^3 and 50 at 128^3: 128^3 to 1e-6 takes
+// 0.4 % longer than in launches of 2048, and would take 0.8 % in 8 ms.
 //
 // Every wait is bounded (kPsPolls polls); a CTA that runs out of them sets
 // SolveCtl::aux[0] and leaves, and the host returns an error.
@@ -48,7 +49,7 @@
 namespace pf {
 
 constexpr int kPsVirt = kMaxRedBlocks / kPsGrid;    // virtual CTAs of one CTA, at most
-constexpr int kPsTurns = 1024, kPsStreamTurns = 4 * kPsTurns;
+constexpr int kPsTurns = 2048, kPsStreamTurns = 4 * kPsTurns;
 constexpr unsigned kPsPolls = 1u << 22;
 constexpr int kPsWarps = PF_TV / 32;                // warps of a virtual CTA
 constexpr int kPsFace = 6 * 64;                     // face values of a slot

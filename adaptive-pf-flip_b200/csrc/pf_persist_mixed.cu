@@ -4,8 +4,10 @@
 // stay on chip, the CTAs hand over the z of their slots' faces as tagged pairs.
 // Roundings, fused multiply-adds and the order of the sums are those of the
 // three kernels per iteration it replaces (pf_pcg.cu), so z and the iteration
-// count have the same bits.  An inner iteration on 51 x 64 x 45 cells: 25 us as
-// three launches, 5.5 us here.
+// count have the same bits.  An inner iteration, three launches and here: 51 x 64
+// x 45 cells (three slots a CTA) 25 and 5.5 us, 704 tiles (five) 25.4 and 8.0, 900
+// (seven) 31.3 and 9.9, 1000 31.5 and 10.1 (BF16 couplings 33.6 and 10.1).  Eight
+// slots are what the partial sums' scratch holds.
 #include <cuda_bf16.h>
 
 #include <algorithm>

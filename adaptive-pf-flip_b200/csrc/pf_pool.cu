@@ -193,7 +193,10 @@ __global__ void k_bump_nslots(int* d_nslots, const int* added) { *d_nslots += *a
 // The four steps above (flags, scan, slots, new size) in one CTA for tile
 // lattices of up to kCommitTiles tiles (152^3 cells): thread t takes tiles
 // kCommitPer t ..., so the scan keeps ascending tile order.  A commit is a chain
-// of six to eight launches of about 2.4 us otherwise, four times a step.
+// of six to eight launches of about 2.4 us otherwise, four times a step.  It pays
+// up to what one CTA holds: P2G of a bubble tank by the chain and by this, 40^3
+// cells 138 and 125 us, 72^3 327 and 311, 104^3 604 and 579, 128^3 1059 and 1036,
+// 152^3 1711 and 1683.
 constexpr int kCommitNT = 1024, kCommitPer = 8, kCommitTiles = kCommitNT * kCommitPer;
 __global__ void __launch_bounds__(kCommitNT) k_commit_small(uint8_t* need, int* tile_slot, int* slot_tile,
                                                             int* d_nslots, int n) {

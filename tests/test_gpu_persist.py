@@ -106,13 +106,13 @@ def test_flexible_pcg_on_ragged_systems_reaches_the_plain_solution(pf, shape, in
 
 
 def test_long_solve_gives_the_bits_of_the_allocation_free_one(pf):
-    """A solve of more iterations than one launch runs (1024), on a system that
+    """A solve of more iterations than one launch runs (2048), on a system that
     lasts that long, against the allocation-free entry point, whose three kernels
     per iteration form the same sums in the same order."""
     import ctypes as C
 
     import torch
-    n, dt, its = 38, 1.0 / 240, 1500  # 125 tiles, all pooled by both entry points
+    n, dt, its = 38, 1.0 / 240, 2500  # 125 tiles, all pooled by both entry points
     sc = pf.scenes.ellipsoid_pressure(n, seed=1)
     pp = pf.PhaseParams(sc["rho_l"], sc["rho_g"])
     g = pf.SparseMacGrid3D(n, n, n, 1.0 / n, max_particles=n ** 3 // 4)
