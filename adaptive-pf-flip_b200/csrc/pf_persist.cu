@@ -32,7 +32,7 @@ struct PsPlain {
   PsBar bar;
   PsPair* faces;  // [2][nslots][6][64]
   unsigned long long tag;
-  int turns;      // iterations of this launch, at most
+  int turns, max_iter;  // iterations of this launch, at most, and of the solve
 };
 
 // ---- everything on chip ---------------------------------------------------
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(PF_TV, 1) k_plain_resident(PsPlain A) {
   const int at_y = ly == 7 ? 128 + fy : ly == 0 ? 192 + fy : -1;
   const int at_z = lz == 7 ? 256 + fz : lz == 0 ? 320 + fz : -1;
 
-  PsScalars sc(A.ctl);
+  PsScalars sc(A.ctl, A.turns);
   double r[U], za[U], dg[U], inv[U], hz[U];  // za: z, and Ap between the two phases
   unsigned live = 0, pinned = 0;
 #pragma unroll
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(PF_TV, 1) k_plain_resident(PsPlain A) {
   const bool writes = (lane & (32 / N - 1)) == 0;
   bool alive = true;
   unsigned long long arrivals = 0;
-  for (int turn = 0; turn < A.turns && !sc.done; ++turn) {
+  for (int turn = 0; !sc.done; ++turn) {
     const int par = turn & 1;
     const unsigned long long tag = A.tag + turn;
     // ---- phase 1
@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(PF_TV, 1) k_plain_resident(PsPlain A) {
     if (!alive) break;
     sc.after_update(S, M);
   }
+  sc.end_launch(A.max_iter);
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (!((live >> u) & 1u)) continue;
@@ -266,7 +267,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
   double* s_x = s_r + (size_t)kr * PF_TV;         // [kx][512]
   int* s_nbr = reinterpret_cast<int*>(s_x + (size_t)kx * PF_TV);  // [k][8]
   uint8_t* s_kind = reinterpret_cast<uint8_t*>(s_nbr + 8 * k);    // [k][512]
-  PsScalars sc(A.ctl);
+  PsScalars sc(A.ctl, A.max_iter - A.ctl->it);  // its loop bound ends the launch
   double* P = A.p0;
   for (int m = half; m < k; m += 2) {
     const int s = c + kPsGrid * m, q = m * PF_TV + l;
@@ -291,7 +292,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_plain_stream(PsPlain A, i
   const bool writes = (lane & (32 / N - 1)) == 0 && own < nvirt;
   bool pend = false, alive = true;
   unsigned long long arrivals = 0;
-  for (int turn = 0; turn < A.turns && !sc.done; ++turn) {
+  // turns count up to a constant, from where leaves A.turns (a bound in a register
+  // changed the allocation of phase 1: 0.5 % at 128^3)
+  for (int turn = kPsTurns - A.turns; turn < kPsTurns && !sc.done; ++turn) {
     const int par = turn & 1;
     const unsigned long long tag = A.tag + turn;
     // ---- direction
@@ -498,10 +501,10 @@ int plain_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
   const bool resident = k <= kResSlots;
   if (!resident && k * ps_slot_bytes() > room) return PF_OK;
   PsPlain a{nslots, std::min(nslots, kMaxRedBlocks), ctx->ctl, kind, nbr, v.x, v.r, v.p, v.z, v.diag, v.cx, v.cy,
-            v.cz, scale, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0, 0};
+            v.cz, scale, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0, 0, max_iter};
   while (!out->done && *launched < max_iter) {
-    a.turns = std::min(check_every > 0 ? check_every : resident ? kPsTurns : kPsStreamTurns / k, max_iter - *launched);
-    a.tag = ctx->ps_tag + 1;
+    a.turns = ps_turns(check_every, resident ? kPsTurns : kPsStreamTurns / k, max_iter - *launched);
+    a.tag = ctx->ps_tag + 1 - (resident ? 0 : kPsTurns - a.turns);  // the tag of turn 0
     ctx->ps_tag += a.turns;
     bool refused = false;
     const int rc = resident ? launch_resident(ctx, a, k, grid, &refused) : launch_stream(ctx, a, k, grid, room, &refused);

@@ -44,6 +44,8 @@
 // SolveCtl::aux[0] and leaves, and the host returns an error.
 #pragma once
 
+#include <algorithm>
+
 #include "pf_solver.cuh"
 
 namespace pf {
@@ -56,6 +58,12 @@ constexpr int kPsFace = 6 * 64;                     // face values of a slot
 
 static_assert(kMaxRedBlocks % kPsGrid == 0, "a CTA must own whole virtual CTAs");
 static_assert(kPsWarps == 16, "half a warp folds one virtual CTA");
+
+// iterations of the next launch: check_every if the caller gives it, else by_time
+inline int ps_turns(int check_every, int by_time, int left) {
+  const int n = check_every > 0 ? std::min(check_every, kPsTurns) : by_time;
+  return std::min(n, left);
+}
 
 // a value and its tag, as one 16-byte access
 __device__ __forceinline__ void ps_store(PsPair* p, double v, unsigned long long tag) {
@@ -260,12 +268,14 @@ __device__ __forceinline__ int halo_cell(int d, int q) {
 }
 
 // The scalars of a solve, advanced alike by every thread of the grid (the
-// rules of finalize_stage, kStagePAp and kStageUpdate).
+// rules of finalize_stage, kStagePAp and kStageUpdate).  A launch ends when done is
+// set: by its last iteration too (a loop bound of its own took a register and 0.04 us
+// of the 7.7 at 64^3), which end_launch takes back while max_iter is not reached.
 struct PsScalars {
   double alpha, beta, rz, res, tol;
-  int it, max_iter, done;
-  __device__ __forceinline__ explicit PsScalars(const SolveCtl* c)
-      : alpha(0.0), beta(c->beta), rz(c->rz), res(c->res), tol(c->tol), it(c->it), max_iter(c->max_iter),
+  int it, stop, done;
+  __device__ __forceinline__ PsScalars(const SolveCtl* c, int turns)
+      : alpha(0.0), beta(c->beta), rz(c->rz), res(c->res), tol(c->tol), it(c->it), stop(c->it + turns),
         done(c->done) {}
   __device__ __forceinline__ void after_pap(double S) {
     if (!isfinite(S)) done = 4;
@@ -277,11 +287,14 @@ struct PsScalars {
     res = M;
     if (!isfinite(M) || !isfinite(S)) done = 4;
     else if (M < tol) done = 1;
-    else if (it >= max_iter) done = 3;
     else {
       beta = S / rz;
       rz = S;
+      if (it >= stop) done = 3;
     }
+  }
+  __device__ __forceinline__ void end_launch(int max_iter) {
+    if (done == 3 && it < max_iter) done = 0;
   }
   __device__ __forceinline__ void store(SolveCtl* c) const {
     c->alpha = alpha;

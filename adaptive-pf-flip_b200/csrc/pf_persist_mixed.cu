@@ -31,7 +31,7 @@ struct PsMixed {
   PsBar bar;
   PsPair* faces;
   unsigned long long tag;
-  int turns;  // iterations of this launch, at most
+  int turns, max_iter;  // iterations of this launch, at most, and of the solve
 };
 
 __device__ __forceinline__ float ld16(const void* a, int is16, size_t i) {
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(PF_TV, 1) k_mixed_resident(PsMixed A) {
   const int at_y = ly == 7 ? 128 + fy : ly == 0 ? 192 + fy : -1;
   const int at_z = lz == 7 ? 256 + fz : lz == 0 ? 320 + fz : -1;
 
-  PsScalars sc(A.ctl);
+  PsScalars sc(A.ctl, A.turns);
   if (A.first) sc.beta = 0.0;
   float e[U], r[U], za[U], dg[U], hz[U];  // za: z, and A'p between the two phases
   unsigned live = 0, pinned = 0, has = 0;  // has: this thread's neighbours across a face exist, 3 bits a slot
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(PF_TV, 1) k_mixed_resident(PsMixed A) {
   const bool writes = (lane & (32 / N - 1)) == 0;
   bool alive = true;
   unsigned long long arrivals = 0;
-  for (int turn = 0; turn < A.turns && !sc.done; ++turn) {
+  for (int turn = 0; !sc.done; ++turn) {
     const int par = turn & 1;
     const unsigned long long tag = A.tag + turn;
     // ---- phase 1: p = z + beta p, A'p
@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(PF_TV, 1) k_mixed_resident(PsMixed A) {
     if (!alive) break;
     sc.after_update(S, M);
   }
+  sc.end_launch(A.max_iter);
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (!((live >> u) & 1u)) continue;
@@ -249,9 +250,9 @@ int mixed_persist(pf_ctx* ctx, int nslots, const uint8_t* kind, const int* nbr, 
   *launched = 0;
   if (nslots <= 0 || ctx->num_sms < kPsGrid || k > kPsVirt) return PF_OK;
   PsMixed a{nslots, std::min(nslots, kMaxRedBlocks), 1, cc16, cp16, ctx->ctl, kind, nbr, e, r, d, p,
-            {c[0], c[1], c[2]}, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0, 0};
+            {c[0], c[1], c[2]}, PsBar{ctx->ps_entries, ctx->ps_counter}, ctx->ps_faces, 0, 0, max_iter};
   while (!out->done && *launched < max_iter) {
-    a.turns = std::min(check_every > 0 ? check_every : kPsTurns, max_iter - *launched);
+    a.turns = ps_turns(check_every, kPsTurns, max_iter - *launched);
     a.tag = ctx->ps_tag + 1;
     ctx->ps_tag += a.turns;
     bool refused = false;
