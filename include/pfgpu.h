@@ -95,7 +95,7 @@ typedef struct {
   int bf16_storage;     /* mixed: 1 store the inner solve's couplings (beta) in BF16; 2 also its search
                            direction */
   int check_every;      /* host convergence poll interval in iterations, the most that one launch of a
-                           persistent kernel runs (0 = default).  The results do not depend on it. */
+                           persistent kernel runs, up to 2048 (0 = default).  The results do not depend on it. */
   int max_refine;       /* unused (kept for the struct layout) */
   double inner_rel_tol; /* mixed / learned FP32: an inner solve stops at max|r| <= inner_rel_tol max|r_0|
                            (0 = default: 1e-3) */
